@@ -27,6 +27,7 @@
 
 #include "fm_common.cuh"
 #include "fm_internal.h"
+#include "fm_mg_cluster.cuh"
 
 namespace fm {
 
@@ -910,9 +911,24 @@ __global__ void k_laplacian(Shape s, const T* __restrict__ p, T* __restrict__ Ap
   }
 }
 
-}  // namespace fm
+// k_pcg_cluster's connection to the solver state
+__device__ __forceinline__ bool pcg_skip(const DevState* st) { return st->dc_done != 0; }  // 0 outside fm_project_dc
+__device__ __forceinline__ double pcg_floor(const DevState* st) { return st->dc_tol; }
+__device__ __forceinline__ void pcg_finish(DevState* st, const PcgOutcome& R) {
+  st->zTr_old = R.zTr;
+  st->tol = R.tol;
+  st->alpha = R.alpha;
+  st->beta = R.beta;
+  st->mean = R.mean;
+  st->pAp = R.pAp;
+  if (R.stepped) st->rTr = R.rTr;
+  st->it = R.it;
+  st->conv = R.conv;
+  st->nonfinite = R.nonfinite;
+  finish_solve(st);
+}
 
-#include "fm_mg_cluster.cuh"
+}  // namespace fm
 
 using namespace fm;
 
@@ -941,57 +957,63 @@ struct fm_mgpcg {
   int lc;                      // levels lc .. L-1 run as one cluster launch (<= 0: per-level launches)
   int nc;                      // CTAs in that cluster
   size_t coarse_smem;
+  ClArgs coarse;               // its geometry
+  ClArgs* d_coarse;
+  int pcg_nc;                  // CTAs of the cluster that runs a whole solve (0: the solve is a sequence of launches)
+  size_t pcg_smem;
+  ClArgs pcg;
+  ClArgs* d_pcg;
   int bf16_hi;                 // levels 1 .. bf16_hi-1 stored in BF16 (0: none)
 };
 
 namespace fm {
 
-// (red, black) cell pairs along the innermost axis of `planes` planes of level s.
+// Picks the finest level lc >= 1 from which the rest of the V-cycle runs as one
+// cluster launch: level lc split into nc <= 8 slabs of an even number of planes,
+// every slab and every deeper level at most 4096 cells (two pairs per thread:
+// beyond that a per-level launch spread over the chip is faster).  lc = -1 when
+// no level qualifies (the V-cycle launches per level).
+constexpr int kCoarseMaxNC = 8;
+constexpr long kCoarseMaxPairs = 2 * kClThreads;
+
 static long coarse_pairs(const Shape& s, int dim, int planes) {
   const long nin = dim == 3 ? s.s2 : s.s1;
   return (long)planes * (dim == 3 ? s.s1 : 1) * ((nin + 1) / 2);
 }
-static long coarse_ring(const Shape& s, int dim, int planes) {
-  return (long)planes * (s.s1 + 2) * (dim == 3 ? s.s2 + 2 : 1);
-}
 
-// Picks the finest level lc >= 1 from which the rest of the V-cycle fits one
-// cluster launch: level lc split into nc <= 8 slabs of an even number of
-// planes, every slab and every deeper level at most kCoarsePPT cell pairs per
-// thread, all of it (zero-ringed z, compact r) within 200 KB of shared memory
-// per CTA.  lc = -1 when no level qualifies (the V-cycle launches per level).
 static void plan_coarse(fm_mgpcg* S, size_t es) {
   S->lc = -1;
   S->nc = 0;
   S->coarse_smem = 0;
   const int dim = S->g.dim;
-  const long max_pairs = (long)kCoarsePPT * kCoarseThreads;
   for (int l = 1; l < S->L - 1; ++l) {
     const Shape t = S->lv[l];
     int nc = kCoarseMaxNC;
     while (nc > 1 && t.s0 % (2 * nc) != 0) nc >>= 1;
-    if (t.s0 % (2 * nc) != 0) continue;
-    const int P = t.s0 / nc;
-    if (coarse_pairs(t, dim, P) > max_pairs) continue;
-    long cells = coarse_ring(t, dim, P + 2) + (long)P * t.s1 * t.s2;
+    if (t.s0 % (2 * nc) != 0 || coarse_pairs(t, dim, t.s0 / nc) > kCoarseMaxPairs) continue;
     bool fits = true;
-    for (int m = l + 1; m < S->L; ++m) {
-      const Shape d = S->lv[m];
-      fits = fits && coarse_pairs(d, dim, d.s0) <= max_pairs;
-      cells += d.size() + coarse_ring(d, dim, d.s0 + 2);
-    }
-    const size_t smem = es * (size_t)cells;
-    if (!fits || smem > 200 * 1024) continue;
+    for (int m = l + 1; m < S->L; ++m) fits = fits && coarse_pairs(S->lv[m], dim, S->lv[m].s0) <= kCoarseMaxPairs;
+    const size_t smem = cl_layout(S->coarse, S->lv, l, l + 1, S->L, dim, es, nc, false, false);
+    if (!fits || smem == 0 || smem > kClMaxSmem) continue;
     S->lc = l;
     S->nc = nc;
     S->coarse_smem = smem;
+    S->coarse.pre_post = S->P.pre_post;
+    S->coarse.bottom = S->P.bottom;
+    S->coarse.bottom_mode = S->P.bottom_mode;
     return;
   }
 }
 
 template <typename T, int D>
 static bool enable_coarse_kernel(size_t smem) {
-  return raise_smem_limit(k_mg_coarse<T, D>, smem);
+  return raise_smem_limit(k_mg_coarse<T, D, DevState>, smem);
+}
+
+template <typename T, int D>
+static void plan_pcg_t(fm_mgpcg* S) {
+  S->pcg_nc = cl_plan_pcg(S->pcg, k_pcg_cluster<T, D, false, DevState*>, S->lv, S->L, S->P, D, sizeof(T), false,
+                          &S->pcg_smem);
 }
 
 static inline unsigned blocks_for(long n, int threads, long cap) {
@@ -1004,40 +1026,8 @@ static inline unsigned blocks_for(long n, int threads, long cap) {
 // Levels lc .. L-1 of the V-cycle as one cluster launch (fm_mg_cluster.cuh).
 template <typename T, int D>
 static void launch_coarse(fm_mgpcg* S, cudaStream_t s) {
-  CoarseArgs a;
-  int off = 0;  // deep levels in CTA 0: compact r, then zero-ringed z
-  for (int l = 0; l < kMaxLevels; ++l) {
-    a.lv[l] = S->lv[l];
-    a.roff[l] = a.zoff[l] = off;
-    if (l > S->lc && l < S->L) {
-      a.zoff[l] = off + (int)S->lv[l].size();
-      off = a.zoff[l] + (int)coarse_ring(S->lv[l], S->g.dim, S->lv[l].s0 + 2);
-    }
-  }
-  a.lc = S->lc;
-  a.L = S->L;
-  a.pre_post = S->P.pre_post;
-  a.bottom = S->P.bottom;
-  a.bottom_mode = S->P.bottom_mode;
-  a.r_top = S->r[S->lc];
-  a.z_top = S->z[S->lc];
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)S->nc, 1, 1);
-  cfg.blockDim = dim3(kCoarseThreads, 1, 1);
-  cfg.dynamicSmemBytes = S->coarse_smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S->nc;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = g_pdl.load(std::memory_order_relaxed) ? 2 : 1;
-  const DevState* st = S->st;
-  cudaLaunchKernelEx(&cfg, k_mg_coarse<T, D>, a, st);
-  count_launch(1);
+  cl_launch(k_mg_coarse<T, D, DevState>, S->nc, S->coarse_smem, s, (const ClArgs*)S->d_coarse, (const T*)S->r[S->lc],
+            (T*)S->z[S->lc], (const DevState*)S->st);
 }
 
 // One V-cycle (apply_preconditioner, 3D/mgpcg.py:187-205) on r[0] -> z[0].
@@ -1293,13 +1283,34 @@ static int capture_solve(fm_mgpcg* S, cudaStream_t s) {
   return FM_OK;
 }
 
+// The outcome of the solve just enqueued on s (a host synchronisation).
+static int read_outcome(fm_mgpcg* S, cudaStream_t s, int* iters, double* rtr) {
+  if (cudaMemcpyAsync(S->h_st, S->st, sizeof(DevState), cudaMemcpyDeviceToHost, s) != cudaSuccess) return FM_ERR_CUDA;
+  if (cudaStreamSynchronize(s) != cudaSuccess) return FM_ERR_CUDA;
+  if (iters) *iters = S->h_st->result_it;
+  if (rtr) *rtr = S->h_st->rTr;
+  if (S->h_st->nonfinite) return FM_ERR_NONFINITE;
+  if (!S->h_st->conv) return FM_ERR_NOT_CONVERGED;
+  return FM_OK;
+}
+
 template <typename T>
 static int run_solve(fm_mgpcg* S, cudaStream_t s, int* iters, double* rtr) {
   const int D = S->g.dim;
   if (stream_capturing(s)) {
     // recorded, not run: no host read of the outcome, no host-checked loop
     if (iters || rtr || S->P.check_every != 0) return FM_ERR_ARG;
-    return capture_solve<T>(S, s);
+    if (!S->pcg_nc) return capture_solve<T>(S, s);
+  }
+  if (S->pcg_nc) {
+    const PcgParams pp{S->P.max_iters, S->P.abs_tol, S->P.rel_tol, S->P.eps};
+    auto go = [&](auto k) { cl_launch(k, S->pcg_nc, S->pcg_smem, s, (const ClArgs*)S->d_pcg, pp, (const T*)S->r[0], (T*)S->x, S->st); };
+    if (D == 3) go(k_pcg_cluster<T, 3, false, DevState*>);
+    else go(k_pcg_cluster<T, 2, false, DevState*>);
+    const int e = check_cuda();
+    if (e) return e;
+    if (S->P.check_every == 0 && !iters && !rtr) return FM_OK;  // asynchronous: outcome via fm_mgpcg_stats
+    return read_outcome(S, s, iters, rtr);
   }
   if (!S->prologue) {
     const int e = build_prologue_graph<T>(S);
@@ -1314,13 +1325,7 @@ static int run_solve(fm_mgpcg* S, cudaStream_t s, int* iters, double* rtr) {
     }
     if (cudaGraphLaunch(S->loop, s) != cudaSuccess) return FM_ERR_CUDA;
     if (!iters && !rtr) return FM_OK;  // asynchronous: outcome via fm_mgpcg_stats
-    if (cudaMemcpyAsync(S->h_st, S->st, sizeof(DevState), cudaMemcpyDeviceToHost, s) != cudaSuccess) return FM_ERR_CUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return FM_ERR_CUDA;
-    if (iters) *iters = S->h_st->result_it;
-    if (rtr) *rtr = S->h_st->rTr;
-    if (S->h_st->nonfinite) return FM_ERR_NONFINITE;
-    if (!S->h_st->conv) return FM_ERR_NOT_CONVERGED;
-    return FM_OK;
+    return read_outcome(S, s, iters, rtr);
   }
   if (!S->chunk) {
     cudaGraph_t graph;
@@ -1399,6 +1404,11 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
   }
   // BF16 storage for the per-level coarse levels 1 .. lc-1 (needs the cluster path)
   S->bf16_hi = (P.coarse_bf16 && S->lc > 1) ? S->lc : 0;
+  // a grid that fits one cluster is solved in one launch (with BF16 levels it keeps those)
+  if (S->bf16_hi == 0) {
+    if (dtype == FM_F32) g->dim == 3 ? plan_pcg_t<float, 3>(S) : plan_pcg_t<float, 2>(S);
+    else g->dim == 3 ? plan_pcg_t<double, 3>(S) : plan_pcg_t<double, 2>(S);
+  }
   for (int l = 0; l < S->L; ++l) {
     const size_t e = (l >= 1 && l < S->bf16_hi) ? sizeof(__nv_bfloat16) : es;
     ok = ok && cudaMalloc(&S->r[l], e * S->lv[l].size()) == cudaSuccess;
@@ -1406,10 +1416,26 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
   }
   const long n0 = S->lv[0].size();
   ok = ok && cudaMalloc(&S->x, es * n0) == cudaSuccess;
-  ok = ok && cudaMalloc(&S->p, es * n0) == cudaSuccess;
-  ok = ok && cudaMalloc(&S->Ap, es * n0) == cudaSuccess;
-  ok = ok && cudaMalloc(&S->part, sizeof(double) * 2 * kRedBlocks) == cudaSuccess;
-  ok = ok && cudaMalloc(&S->st, sizeof(DevState)) == cudaSuccess;
+  if (!S->pcg_nc) {  // a cluster solve keeps p and A p in shared memory
+    ok = ok && cudaMalloc(&S->p, es * n0) == cudaSuccess;
+    ok = ok && cudaMalloc(&S->Ap, es * n0) == cudaSuccess;
+  }
+  // partials, state and the cluster geometries in one allocation
+  struct Small {
+    double part[2 * kRedBlocks];
+    ClArgs coarse, pcg;
+    DevState st;
+  };
+  Small* small = nullptr;
+  ok = ok && cudaMalloc((void**)&small, sizeof(Small)) == cudaSuccess;
+  if (ok) {
+    S->part = small->part;
+    S->st = &small->st;
+    S->d_coarse = &small->coarse;
+    S->d_pcg = &small->pcg;
+    ClArgs both[2] = {S->coarse, S->pcg};
+    ok = cudaMemcpy(S->d_coarse, both, sizeof(both), cudaMemcpyHostToDevice) == cudaSuccess;
+  }
   ok = ok && cudaMallocHost(&S->h_st, sizeof(DevState)) == cudaSuccess;
   ok = ok && cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) == cudaSuccess;
   if (ok) ok = cudaMemset(S->st, 0, sizeof(DevState)) == cudaSuccess;
@@ -1446,8 +1472,7 @@ int fm_mgpcg_destroy(fm_mgpcg* S) {
   if (S->x) cudaFree(S->x);
   if (S->p) cudaFree(S->p);
   if (S->Ap) cudaFree(S->Ap);
-  if (S->part) cudaFree(S->part);
-  if (S->st) cudaFree(S->st);
+  if (S->part) cudaFree(S->part);  // and the state and the cluster geometries with it
   if (S->h_st) cudaFreeHost(S->h_st);
   if (S->chunk) cudaGraphExecDestroy(S->chunk);
   if (S->prologue) cudaGraphExecDestroy(S->prologue);

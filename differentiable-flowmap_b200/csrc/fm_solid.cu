@@ -16,10 +16,11 @@
 // atomics), so the V-cycle equals the oracle's bit for bit.  PCG inner
 // products are fixed-grid FP64 reductions.
 //
-// B200 mapping.  The hierarchy is small next to the flow-map state (256^2:
-// 0.5 MB per level), so the levels are plain global arrays and every step is a
-// grid-stride kernel; the coarsest levels that fit 96 KB of shared memory
-// (down-sweeps, bottom, up-sweeps) run in one CTA out of shared memory.  The PCG loop keeps its
+// B200 mapping.  A grid whose solver state fits one thread-block cluster (up to
+// 16 CTAs' shared memory) is solved in one launch (k_pcg_cluster).  Otherwise
+// the levels are plain global arrays and every step is a grid-stride kernel;
+// the coarsest levels that fit 96 KB of shared memory (down-sweeps, bottom,
+// up-sweeps) run in one CTA out of shared memory.  The PCG loop keeps its
 // scalars (alpha, beta, the inner products, a done flag) on the device: every
 // kernel of an iteration returns at once after convergence, so the host only
 // polls the flag every check_every iterations (a chunk of iterations captured
@@ -38,6 +39,7 @@
 
 #include "fm_common.cuh"
 #include "fm_internal.h"
+#include "fm_mg_cluster.cuh"
 
 namespace fm {
 namespace solid {
@@ -87,7 +89,7 @@ __global__ void k_loop_init(cudaGraphConditionalHandle h, const State* st) {
   cudaGraphSetConditional(h, st->done ? 0u : 1u);
 }
 
-__global__ void k_stats(const State* st, Stats* out) {
+__device__ __forceinline__ void add_stats(const State* st, Stats* out) {
   const bool nf = !isfinite(st->rtr);
   out->solves += 1;
   out->iterations += st->iters;
@@ -96,6 +98,30 @@ __global__ void k_stats(const State* st, Stats* out) {
   out->last_iters = st->iters;
   if (st->iters > out->max_iters_seen) out->max_iters_seen = st->iters;
   out->last_rtr = st->rtr;
+}
+__global__ void k_stats(const State* st, Stats* out) { add_stats(st, out); }
+
+// k_pcg_cluster's connection to the solver state: the whole outcome of a solve
+// and its statistics are written when it ends.
+struct Ctx {
+  State* st;
+  Stats* stats;
+};
+__device__ __forceinline__ bool pcg_skip(const Ctx&) { return false; }
+__device__ __forceinline__ double pcg_floor(const Ctx&) { return 0.0; }
+__device__ __forceinline__ void pcg_finish(const Ctx& c, const PcgOutcome& R) {
+  State* st = c.st;
+  st->old_zr = R.zTr;
+  st->tol = R.tol;
+  st->rtr = R.stepped ? R.rTr : 0.0;
+  st->pAp = R.pAp;
+  st->alpha = R.alpha;
+  st->beta = R.beta;
+  st->mean = R.mean;
+  st->done = 1;
+  st->iters = R.it;
+  st->converged = R.conv;
+  add_stats(st, c.stats);
 }
 
 __device__ __forceinline__ void idx3(const Shape& s, long q, int* I) {
@@ -147,6 +173,38 @@ __global__ void k_downsample(Shape sf, const uint8_t* __restrict__ ff, Shape sc,
       for (int d1 = 0; d1 < 2; ++d1)
         for (int d2 = 0; d2 < (D == 3 ? 2 : 1); ++d2) any |= ff[sf.idx(2 * I[0] + d0, 2 * I[1] + d1, D == 3 ? 2 * I[2] + d2 : 0)];
     fc[q] = any;
+  }
+}
+
+// The obstacle mask of a level as the cluster solve reads it: one word per pair
+// of cells (2m, 2m + 1) of a row, holding per colour c at bit 8c the in-domain
+// fluid neighbours (+i -i +j -j +k -k; in 2D the last two are +j -j) and, at
+// bit 6, whether the cell is fluid (fm_mg_cluster.cuh).
+template <int D>
+__global__ void k_pack_mask(Shape s, const uint8_t* __restrict__ fl, uint16_t* __restrict__ out) {
+  const int nin = D == 3 ? s.s2 : s.s1, M = (nin + 1) / 2;
+  const long rows = (long)s.s0 * (D == 3 ? s.s1 : 1);
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < rows * M; e += (long)gridDim.x * blockDim.x) {
+    const long row = e / M;
+    const int m = (int)(e - row * M);
+    unsigned w = 0;
+    for (int h = 0; h < 2; ++h) {
+      const int k = 2 * m + h;
+      if (k >= nin) continue;
+      const long q = row * nin + k;
+      if (!fl[q]) continue;
+      int I[3];
+      idx3(s, q, I);
+      unsigned b = 64;
+      for (int a = 0; a < D; ++a) {
+        const long st = stride_of(s, a);
+        const int sh = a == D - 1 ? 4 : 2 * a;
+        if (I[a] < axis_len(s, a) - 1 && fl[q + st]) b |= 1u << sh;
+        if (I[a] > 0 && fl[q - st]) b |= 2u << sh;
+      }
+      w |= b << (8 * ((I[0] + I[1] + I[2]) & 1));
+    }
+    out[e] = (uint16_t)w;
   }
 }
 
@@ -451,64 +509,62 @@ __global__ void k_init(long n, const T* __restrict__ b, T k, T* __restrict__ r, 
 }
 
 // ----------------------------------------------------------------- projection
-// zero the domain walls and the faces of solid cells
-template <typename T, int D>
-__global__ void k_bc(fm_grid g, int c, T* __restrict__ u, const uint8_t* __restrict__ fl) {
-  const Shape fs = face_shape(g, c), cs = cell_shape(g);
-  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < fs.size(); q += (long)gridDim.x * blockDim.x) {
-    int I[3];
-    idx3(fs, q, I);
-    bool zero = I[c] == 0 || I[c] == axis_len(fs, c) - 1;
-    if (!zero && I[c] < axis_len(cs, c) && !fl[cs.idx(I[0], I[1], I[2])]) zero = true;
-    if (!zero && I[c] >= 1) {
-      int J[3] = {I[0], I[1], I[2]};
-      J[c] -= 1;
-      if (!fl[cs.idx(J[0], J[1], J[2])]) zero = true;
-    }
-    if (zero) u[q] = (T)0;
-  }
+// A face that the boundary conditions zero: a domain wall, or a face of a solid cell.
+template <int D>
+__device__ __forceinline__ bool face_closed(const Shape& cs, int c, const int* I, const uint8_t* __restrict__ fl) {
+  if (I[c] == 0 || I[c] == axis_len(cs, c)) return true;
+  const long q = cs.idx(I[0], I[1], I[2]);
+  return !fl[q] || !fl[q - stride_of(cs, c)];
 }
 
+// Front of a projection in one pass: r = -div(u) of the fluid cells with the
+// closed faces taken as zero (u itself is zeroed there by k_project_back), x =
+// p = 0.  (One launch instead of five: the passes are bound by launch latency.)
 template <typename T, int D>
-__global__ void k_div(fm_grid g, const T* __restrict__ ux, const T* __restrict__ uy, const T* __restrict__ uz,
-                      const uint8_t* __restrict__ fl, T* __restrict__ div) {
+__global__ void k_project_front(fm_grid g, const T* __restrict__ ux, const T* __restrict__ uy,
+                                const T* __restrict__ uz, const uint8_t* __restrict__ fl, T* __restrict__ r,
+                                T* __restrict__ x, T* __restrict__ p) {
+  pdl_begin();
   const Shape cs = cell_shape(g);
   const T* u[3] = {ux, uy, uz};
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < cs.size(); q += (long)gridDim.x * blockDim.x) {
-    if (!fl[q]) {
-      div[q] = (T)0;
-      continue;
-    }
-    int I[3];
-    idx3(cs, q, I);
     T acc = (T)0;
+    if (fl[q]) {
+      int I[3];
+      idx3(cs, q, I);
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-      const Shape fs = face_shape(g, c);
-      int J[3] = {I[0], I[1], I[2]};
-      const T vl = u[c][fs.idx(J[0], J[1], J[2])];
-      J[c] += 1;
-      const T vr = u[c][fs.idx(J[0], J[1], J[2])];
-      acc = c == 0 ? rn_sub(vr, vl) : rn_sub(rn_add(acc, vr), vl);
+      for (int c = 0; c < D; ++c) {
+        const Shape fs = face_shape(g, c);
+        int J[3] = {I[0], I[1], I[2]};
+        const T vl = face_closed<D>(cs, c, J, fl) ? (T)0 : u[c][fs.idx(J[0], J[1], J[2])];
+        J[c] += 1;
+        const T vr = face_closed<D>(cs, c, J, fl) ? (T)0 : u[c][fs.idx(J[0], J[1], J[2])];
+        acc = c == 0 ? rn_sub(vr, vl) : rn_sub(rn_add(acc, vr), vl);
+      }
     }
-    div[q] = acc;
+    r[q] = acc * (T)-1;
+    x[q] = (T)0;
+    p[q] = (T)0;
   }
 }
 
-// u -= p(I) - p(I - e_c), p = 0 outside (the walls are zeroed by the next k_bc)
+// Back: u -= x(I) - x(I - e_c), closed faces zero.
 template <typename T, int D>
-__global__ void k_grad(fm_grid g, int c, T* __restrict__ u, const T* __restrict__ p) {
+__global__ void k_project_back(fm_grid g, const T* __restrict__ x, const uint8_t* __restrict__ fl, T* ux, T* uy,
+                               T* uz) {
+  pdl_begin();
+  const int c = blockIdx.y;
   const Shape fs = face_shape(g, c), cs = cell_shape(g);
+  T* u = pick3(ux, uy, uz, c);
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < fs.size(); q += (long)gridDim.x * blockDim.x) {
     int I[3];
     idx3(fs, q, I);
-    T pr = (T)0, pl = (T)0;
-    if (I[c] < axis_len(cs, c)) pr = p[cs.idx(I[0], I[1], I[2])];
-    if (I[c] >= 1) {
-      I[c] -= 1;
-      pl = p[cs.idx(I[0], I[1], I[2])];
+    if (face_closed<D>(cs, c, I, fl)) {
+      u[q] = (T)0;
+      continue;
     }
-    u[q] = rn_sub(u[q], rn_sub(pr, pl));
+    const long pc = cs.idx(I[0], I[1], I[2]);
+    u[q] = rn_sub(u[q], rn_sub(x[pc], x[pc - stride_of(cs, c)]));
   }
 }
 
@@ -571,7 +627,8 @@ struct fm_solid {
   void* r[16];
   void* z[16];
   uint8_t* fl[16];
-  void *x, *p, *Ap, *div;
+  uint16_t* msk[16];  // packed masks of the cluster solve
+  void *x, *p, *Ap;
   double* part;
   fm::solid::State* st;
   fm::solid::State* st_host;  // pinned
@@ -584,6 +641,11 @@ struct fm_solid {
   // device mode (check_every == 0): a graph with a conditional WHILE node
   cudaGraphExec_t loop;
   long long loop_kernels;  // kernels per loop body
+  // a grid that fits one cluster is solved in one launch (0: a sequence of launches)
+  int pcg_nc;
+  size_t pcg_smem;
+  fm::ClArgs pcg;
+  fm::ClArgs* d_pcg;
 };
 
 namespace fm {
@@ -800,26 +862,46 @@ int device_loop(fm_solid* S, cudaStream_t s, bool capturing) {
   return FM_OK;
 }
 
+// The outcome of the solve just enqueued on s (a host synchronisation).
+inline int read_outcome(fm_solid* S, cudaStream_t s, int* iters, double* rtr) {
+  if (cudaMemcpyAsync(S->st_host, S->st, sizeof(State), cudaMemcpyDeviceToHost, s) != cudaSuccess) return FM_ERR_CUDA;
+  if (cudaStreamSynchronize(s) != cudaSuccess) return FM_ERR_CUDA;
+  if (iters) *iters = S->st_host->iters;
+  if (rtr) *rtr = S->st_host->rtr;
+  const int cst = check_cuda();
+  if (cst) return cst;
+  if (!isfinite(S->st_host->rtr)) return FM_ERR_NONFINITE;
+  return S->st_host->converged ? FM_OK : FM_ERR_NOT_CONVERGED;
+}
+
+// Solve from the right-hand side in r[0], x = p = 0 on entry; the solution in S->x.
+// check_every == 0: on the device (capturable into a caller's graph when no
+// outcome is read back); otherwise the host reads the outcome, polling it every
+// check_every iterations where the solve is a sequence of launches, which
+// cannot be recorded.
 template <typename T, int D>
-int solve(fm_solid* S, const void* b, double k, void* x, cudaStream_t s, int* iters, double* rtr) {
-  // check_every == 0: device-side loop (capturable into a caller's graph when
-  // no outcome is read back); otherwise the host polls every check_every
-  // iterations, which cannot be recorded
+int solve(fm_solid* S, void* x, cudaStream_t s, int* iters, double* rtr) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) return FM_ERR_CUDA;
   const bool capturing = cs != cudaStreamCaptureStatusNone;
   const bool device = S->P.check_every == 0;
   if (capturing && (!device || iters || rtr)) return FM_ERR_ARG;
   const long n = S->sh[0].size();
+  if (S->pcg_nc) {
+    const PcgParams pp{S->P.max_iters, S->P.abs_tol, S->P.rel_tol, S->P.eps};
+    cl_launch(k_pcg_cluster<T, D, true, Ctx>, S->pcg_nc, S->pcg_smem, s, (const ClArgs*)S->d_pcg, pp, (const T*)S->r[0], (T*)S->x,
+              Ctx{S->st, S->stats});
+    if (x != nullptr && x != S->x) cudaMemcpyAsync(x, S->x, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
+    if (device && !iters && !rtr) return check_cuda();
+    return read_outcome(S, s, iters, rtr);
+  }
   launch(k_state_init, 1, 1, 0, s, S->st, S->P.max_iters, S->P.abs_tol, S->P.rel_tol, S->P.eps);
   State* st = S->st;
   T* r = (T*)S->r[0];
   T* z = (T*)S->z[0];
   T* p = (T*)S->p;
-  T* xs = (T*)S->x;
   const uint8_t* fl = S->fl[0];
   const unsigned nb = blocks_for(n);
-  launch(k_init<T>, nb, kThreads, 0, s, n, (const T*)b, (T)k, r, xs, p);
   // recenter, precondition, p = z, zTr
   launch(k_dot<T>, kRedBlocks, kThreads, 0, s, n, (const T*)r, (const T*)nullptr, (const uint8_t*)nullptr, S->part,
          (const State*)st);
@@ -836,14 +918,7 @@ int solve(fm_solid* S, const void* b, double k, void* x, cudaStream_t s, int* it
     launch(k_stats, 1, 1, 0, s, (const State*)st, S->stats);
     if (x != nullptr && x != S->x) cudaMemcpyAsync(x, S->x, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
     if (!iters && !rtr) return check_cuda();  // asynchronous: the outcome goes to fm_solid_stats
-    if (cudaMemcpyAsync(S->st_host, st, sizeof(State), cudaMemcpyDeviceToHost, s) != cudaSuccess) return FM_ERR_CUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return FM_ERR_CUDA;
-    if (iters) *iters = S->st_host->iters;
-    if (rtr) *rtr = S->st_host->rtr;
-    const int cst = check_cuda();
-    if (cst) return cst;
-    if (!isfinite(S->st_host->rtr)) return FM_ERR_NONFINITE;
-    return S->st_host->converged ? FM_OK : FM_ERR_NOT_CONVERGED;
+    return read_outcome(S, s, iters, rtr);
   }
   const int every = S->P.check_every;
   if (!S->chunk) {
@@ -869,33 +944,64 @@ int solve(fm_solid* S, const void* b, double k, void* x, cudaStream_t s, int* it
     if (S->st_host->done) break;
   }
   launch(k_stats, 1, 1, 0, s, (const State*)st, S->stats);
-  if (cudaMemcpyAsync(S->st_host, st, sizeof(State), cudaMemcpyDeviceToHost, s) != cudaSuccess) return FM_ERR_CUDA;
-  if (cudaStreamSynchronize(s) != cudaSuccess) return FM_ERR_CUDA;
   if (x != nullptr && x != S->x) cudaMemcpyAsync(x, S->x, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
-  if (iters) *iters = S->st_host->iters;
-  if (rtr) *rtr = S->st_host->rtr;
-  const int cst = check_cuda();
-  if (cst) return cst;
-  if (!isfinite(S->st_host->rtr)) return FM_ERR_NONFINITE;
-  return S->st_host->converged ? FM_OK : FM_ERR_NOT_CONVERGED;
+  return read_outcome(S, s, iters, rtr);
 }
 
 template <typename T, int D>
 int project(fm_solid* S, void* const* u, void* p_out, cudaStream_t s, int* iters, double* rtr) {
   const fm_grid& g = S->g;
-  for (int c = 0; c < D; ++c)
-    launch(k_bc<T, D>, blocks_for(face_shape(g, c).size()), kThreads, 0, s, g, c, (T*)u[c], (const uint8_t*)S->fl[0]);
-  launch(k_div<T, D>, blocks_for(S->sh[0].size()), kThreads, 0, s, g, (const T*)u[0], (const T*)u[1],
-         (const T*)(D == 3 ? u[2] : nullptr), (const uint8_t*)S->fl[0], (T*)S->div);
-  const int st = solve<T, D>(S, S->div, -1.0, nullptr, s, iters, rtr);
+  T* uz = (T*)(D == 3 ? u[2] : nullptr);
+  const uint8_t* fl = S->fl[0];
+  launch_pdl(k_project_front<T, D>, blocks_for(S->sh[0].size()), kThreads, 0, s, g, (const T*)u[0], (const T*)u[1],
+             (const T*)uz, fl, (T*)S->r[0], (T*)S->x, (T*)S->p);
+  const int st = solve<T, D>(S, nullptr, s, iters, rtr);
   if (st != FM_OK && st != FM_ERR_NOT_CONVERGED && st != FM_ERR_NONFINITE) return st;
-  for (int c = 0; c < D; ++c) {
-    launch(k_grad<T, D>, blocks_for(face_shape(g, c).size()), kThreads, 0, s, g, c, (T*)u[c], (const T*)S->x);
-    launch(k_bc<T, D>, blocks_for(face_shape(g, c).size()), kThreads, 0, s, g, c, (T*)u[c], (const uint8_t*)S->fl[0]);
-  }
+  long nf = 0;
+  for (int c = 0; c < D; ++c) nf = face_shape(g, c).size() > nf ? face_shape(g, c).size() : nf;
+  launch_pdl(k_project_back<T, D>, dim3(blocks_for(nf), D), kThreads, 0, s, g, (const T*)S->x, fl, (T*)u[0], (T*)u[1],
+             uz);
   if (p_out) cudaMemcpyAsync(p_out, S->x, S->sh[0].size() * sizeof(T), cudaMemcpyDeviceToDevice, s);
   const int cst = check_cuda();
   return cst ? cst : st;
+}
+
+template <typename T, int D>
+int solve_rhs(fm_solid* S, const void* b, void* x, cudaStream_t s, int* iters, double* rtr) {
+  const long n = S->sh[0].size();
+  launch(k_init<T>, blocks_for(n), kThreads, 0, s, n, (const T*)b, (T)1, (T*)S->r[0], (T*)S->x, (T*)S->p);
+  return solve<T, D>(S, x, s, iters, rtr);
+}
+
+}  // namespace solid
+}  // namespace fm
+
+namespace fm {
+namespace solid {
+
+// The packed masks of every level, from the fluid flags (cluster solves only).
+static void pack_masks(fm_solid* S, cudaStream_t s) {
+  if (!S->pcg_nc) return;
+  for (int l = 0; l < S->levels; ++l) {
+    const unsigned nb = blocks_for(S->sh[l].size());
+    if (S->dim == 2) launch(k_pack_mask<2>, nb, kThreads, 0, s, S->sh[l], (const uint8_t*)S->fl[l], S->msk[l]);
+    else launch(k_pack_mask<3>, nb, kThreads, 0, s, S->sh[l], (const uint8_t*)S->fl[l], S->msk[l]);
+  }
+}
+
+template <typename T, int D>
+static bool plan_cluster(fm_solid* S) {
+  S->pcg_nc = cl_plan_pcg(S->pcg, k_pcg_cluster<T, D, true, Ctx>, S->sh, S->levels, S->P, D, sizeof(T), true,
+                          &S->pcg_smem);
+  bool ok = true;
+  for (int l = 0; S->pcg_nc && l < S->levels; ++l) {
+    const Shape& sh = S->sh[l];
+    const long pairs = (long)sh.s0 * (D == 3 ? sh.s1 : 1) * (((D == 3 ? sh.s2 : sh.s1) + 1) / 2);
+    ok = ok && cudaMalloc((void**)&S->msk[l], sizeof(uint16_t) * pairs) == cudaSuccess;
+    S->pcg.msk[l] = S->msk[l];
+  }
+  if (ok && S->pcg_nc) ok = (S->d_pcg = cl_upload(S->pcg)) != nullptr;
+  return ok;
 }
 
 }  // namespace solid
@@ -909,12 +1015,13 @@ int fm_solid_destroy(fm_solid* S) {
     cudaFree(S->r[l]);
     cudaFree(S->z[l]);
     cudaFree(S->fl[l]);
+    cudaFree(S->msk[l]);
   }
   cudaFree(S->x);
   cudaFree(S->p);
   cudaFree(S->Ap);
-  cudaFree(S->div);
   cudaFree(S->part);
+  cudaFree(S->d_pcg);
   cudaFree(S->st);
   cudaFree(S->stats);
   if (S->st_host) cudaFreeHost(S->st_host);
@@ -939,6 +1046,7 @@ int fm_solid_set_mask(fm_solid* S, const float* mask, void* stream) {
       fm::launch(k_downsample<3>, blocks_for(S->sh[l].size()), kThreads, 0, s, S->sh[l - 1], (const uint8_t*)S->fl[l - 1],
                  S->sh[l], S->fl[l]);
   }
+  pack_masks(S, s);
   return fm::check_cuda();
 }
 
@@ -972,7 +1080,7 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
   }
   const long n = S->sh[0].size();
   ok = ok && cudaMalloc(&S->x, n * es) == cudaSuccess && cudaMalloc(&S->p, n * es) == cudaSuccess &&
-       cudaMalloc(&S->Ap, n * es) == cudaSuccess && cudaMalloc(&S->div, n * es) == cudaSuccess &&
+       cudaMalloc(&S->Ap, n * es) == cudaSuccess &&
        cudaMalloc((void**)&S->part, solid::kRedBlocks * sizeof(double)) == cudaSuccess &&
        cudaMalloc((void**)&S->st, sizeof(solid::State)) == cudaSuccess &&
        cudaMallocHost((void**)&S->st_host, sizeof(solid::State)) == cudaSuccess &&
@@ -980,6 +1088,10 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
        cudaMallocHost((void**)&S->stats_host, sizeof(solid::Stats)) == cudaSuccess &&
        cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) == cudaSuccess;
   if (ok) ok = cudaMemset(S->stats, 0, sizeof(solid::Stats)) == cudaSuccess;
+  if (ok) {
+    if (dtype == FM_F32) ok = g->dim == 2 ? solid::plan_cluster<float, 2>(S) : solid::plan_cluster<float, 3>(S);
+    else ok = g->dim == 2 ? solid::plan_cluster<double, 2>(S) : solid::plan_cluster<double, 3>(S);
+  }
   if (!ok) {
     fm_solid_destroy(S);
     return FM_ERR_CUDA;
@@ -1000,6 +1112,7 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
     }
   } else {
     for (int l = 0; l < P.levels; ++l) cudaMemset(S->fl[l], 1, S->sh[l].size());
+    solid::pack_masks(S, nullptr);
   }
   *out = S;
   return check_cuda();
@@ -1057,8 +1170,8 @@ int fm_solid_solve(fm_solid* S, const void* b, void* x, void* stream, int* iters
   if (!S || !b || !x) return FM_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (S->dtype == FM_F32)
-    return S->dim == 2 ? solve<float, 2>(S, b, 1.0, x, s, iters, rtr) : solve<float, 3>(S, b, 1.0, x, s, iters, rtr);
-  return S->dim == 2 ? solve<double, 2>(S, b, 1.0, x, s, iters, rtr) : solve<double, 3>(S, b, 1.0, x, s, iters, rtr);
+    return S->dim == 2 ? solve_rhs<float, 2>(S, b, x, s, iters, rtr) : solve_rhs<float, 3>(S, b, x, s, iters, rtr);
+  return S->dim == 2 ? solve_rhs<double, 2>(S, b, x, s, iters, rtr) : solve_rhs<double, 3>(S, b, x, s, iters, rtr);
 }
 
 int fm_solid_project(fm_solid* S, void* ux, void* uy, void* uz, void* p_out, void* stream, int* iters, double* rtr) {
