@@ -188,11 +188,11 @@ FM_BF16 = 2
 
 def dtype_code(t: torch.dtype, storage: bool = False) -> int:
     """FM_F32/FM_F64 for compute entry points; FM_BF16 too for storage (fm_convert)."""
-    if t == torch.float32:
+    if t is torch.float32:
         return FM_F32
-    if t == torch.float64:
+    if t is torch.float64:
         return FM_F64
-    if storage and t == torch.bfloat16:
+    if storage and t is torch.bfloat16:
         return FM_BF16
     raise FlowmapError(7, f"dtype {t}")
 
@@ -201,16 +201,19 @@ def ptr(t):
     """Device pointer of a contiguous CUDA tensor (None passes NULL)."""
     if t is None:
         return None
+    if t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
     if not t.is_cuda:
         raise FlowmapError(2, "tensor is not on a CUDA device (no CPU fallback)")
-    if not t.is_contiguous():
-        raise FlowmapError(2, "tensor must be contiguous")
-    return t.data_ptr()
+    raise FlowmapError(2, "tensor must be contiguous")
 
 
 def stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """The raw stream: the given one's, else the current device's current stream (read
+    without building a Stream object, which costs more than a kernel launch)."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def header_symbols(path: str = HEADER_PATH):

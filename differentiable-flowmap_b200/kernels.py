@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass
+from functools import cached_property
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -35,6 +36,20 @@ class GridSpec:
         s[c] += 1
         return tuple(s)
 
+    # What every call needs of the grid, built once per GridSpec: a launch of a small
+    # grid's kernel is shorter than the Python that prepares it.
+    @cached_property
+    def _cgrid(self) -> _lib.Grid:
+        return self.c_grid()
+
+    @property
+    def _ref(self):
+        return C.byref(self._cgrid)
+
+    @cached_property
+    def _faces(self) -> Tuple[Tuple[int, ...], ...]:
+        return tuple(self.face_shape(c) for c in range(self.dim))
+
     @property
     def ncell(self) -> int:
         n = 1
@@ -61,8 +76,8 @@ class GridSpec:
 
 
 def _mac3(u):
-    u = list(u) if u is not None else []
-    return [ptr(x) for x in u] + [None] * (3 - len(u))
+    p = [ptr(x) for x in u] if u is not None else []
+    return p if len(p) == 3 else p + [None] * (3 - len(p))
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -70,11 +85,12 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _chk_mac(g: GridSpec, u, name):
-    if len(u) != g.dim:
+    faces = g._faces
+    if len(u) != len(faces):
         raise _lib.FlowmapError(2, f"{name}: expected {g.dim} components")
-    for c, x in enumerate(u):
-        if tuple(x.shape) != g.face_shape(c):
-            raise _lib.FlowmapError(1, f"{name}[{c}] has shape {tuple(x.shape)}, expected {g.face_shape(c)}")
+    for c, (x, want) in enumerate(zip(u, faces)):
+        if x.shape != want:
+            raise _lib.FlowmapError(1, f"{name}[{c}] has shape {tuple(x.shape)}, expected {want}")
 
 
 def _chk_vec(g: GridSpec, t, face, name):
@@ -86,13 +102,13 @@ def _chk_vec(g: GridSpec, t, face, name):
 def advect_u_grid(g: GridSpec, rk: int, dx: float, dt: float, u0, u1, u2, stream=None):
     for n, u in (("u0", u0), ("u1", u1), ("u2", u2)):
         _chk_mac(g, u, n)
-    check(_lib.lib().fm_advect_u_grid(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
+    check(_lib.lib().fm_advect_u_grid(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
                                       *_mac3(u2), stream_ptr(stream)), "fm_advect_u_grid")
 
 
 def advect_scalar_grid(g: GridSpec, rk: int, dx: float, dt: float, u0, s1, s2, stream=None):
     _chk_mac(g, u0, "u0")
-    check(_lib.lib().fm_advect_scalar_grid(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1), ptr(s2),
+    check(_lib.lib().fm_advect_scalar_grid(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1), ptr(s2),
                                            stream_ptr(stream)), "fm_advect_scalar_grid")
 
 
@@ -100,7 +116,7 @@ def advect_u_grid_pair(g: GridSpec, rk: int, dx: float, dt: float, u0, u1, u2, v
     """Two advect_u_grid calls sharing u0/rk/dt, with one backtrace per node."""
     for n, u in (("u0", u0), ("u1", u1), ("u2", u2), ("v1", v1), ("v2", v2)):
         _chk_mac(g, u, n)
-    check(_lib.lib().fm_advect_u_grid_pair(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
+    check(_lib.lib().fm_advect_u_grid_pair(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
                                            *_mac3(u2), *_mac3(v1), *_mac3(v2), stream_ptr(stream)),
           "fm_advect_u_grid_pair")
 
@@ -108,7 +124,7 @@ def advect_u_grid_pair(g: GridSpec, rk: int, dx: float, dt: float, u0, u1, u2, v
 def advect_scalar_grid_pair(g: GridSpec, rk: int, dx: float, dt: float, u0, s1, s2, t1, t2, stream=None):
     """Two advect_scalar_grid calls sharing u0/rk/dt, with one backtrace per cell."""
     _chk_mac(g, u0, "u0")
-    check(_lib.lib().fm_advect_scalar_grid_pair(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1),
+    check(_lib.lib().fm_advect_scalar_grid_pair(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1),
                                                 ptr(s2), ptr(t1), ptr(t2), stream_ptr(stream)),
           "fm_advect_scalar_grid_pair")
 
@@ -118,28 +134,26 @@ def rk_grid(g: GridSpec, rk: int, dx: float, dt: float, face: int, psi, T, u, st
     _chk_vec(g, psi, face, "psi")
     if T is not None:
         _chk_vec(g, T, face, "T")
-    check(_lib.lib().fm_rk_grid(C.byref(g.c_grid()), _dt(psi), rk, dx, dt, face, ptr(psi), ptr(T), *_mac3(u),
+    check(_lib.lib().fm_rk_grid(g._ref, _dt(psi), rk, dx, dt, face, ptr(psi), ptr(T), *_mac3(u),
                                 stream_ptr(stream)), "fm_rk_grid")
 
 
 def march_map(g: GridSpec, rk: int, dx: float, dt: float, psi_c, psi_f, T_f, u, stream=None):
     _chk_mac(g, u, "u")
-    ps = list(psi_f) + [None] * (3 - g.dim)
-    ts = list(T_f) + [None] * (3 - g.dim)
-    check(_lib.lib().fm_march_map(C.byref(g.c_grid()), _dt(u[0]), rk, dx, dt, ptr(psi_c), ptr(ps[0]), ptr(ts[0]),
-                                  ptr(ps[1]), ptr(ts[1]), ptr(ps[2]), ptr(ts[2]), *_mac3(u), stream_ptr(stream)),
-          "fm_march_map")
+    ps, ts = _mac3(psi_f), _mac3(T_f)
+    check(_lib.lib().fm_march_map(g._ref, _dt(u[0]), rk, dx, dt, ptr(psi_c), ps[0], ts[0], ps[1], ts[1], ps[2], ts[2],
+                                  *_mac3(u), stream_ptr(stream)), "fm_march_map")
 
 
 def pullback_u(g: GridSpec, dx: float, u0, out, T_f, psi_f, alpha=1.0, beta=0.0, base=None, stream=None):
     _chk_mac(g, u0, "u0")
     _chk_mac(g, out, "out")
-    check(_lib.lib().fm_pullback_u(C.byref(g.c_grid()), _dt(u0[0]), dx, *_mac3(u0), *_mac3(out), *_mac3(T_f),
+    check(_lib.lib().fm_pullback_u(g._ref, _dt(u0[0]), dx, *_mac3(u0), *_mac3(out), *_mac3(T_f),
                                    *_mac3(psi_f), alpha, beta, *_mac3(base), stream_ptr(stream)), "fm_pullback_u")
 
 
 def pullback_scalar(g: GridSpec, dx: float, s0, out, psi, alpha=1.0, beta=0.0, base=None, stream=None):
-    check(_lib.lib().fm_pullback_scalar(C.byref(g.c_grid()), _dt(s0), dx, ptr(s0), ptr(out), ptr(psi), alpha, beta,
+    check(_lib.lib().fm_pullback_scalar(g._ref, _dt(s0), dx, ptr(s0), ptr(out), ptr(psi), alpha, beta,
                                         ptr(base), stream_ptr(stream)), "fm_pullback_scalar")
 
 
@@ -153,7 +167,7 @@ def advect_scalar_grid_adj(g: GridSpec, rk: int, dx: float, dt: float, u0, s1, g
                            stream=None):
     """g_u0 += dL/du0, g_s1 += dL/ds1 for s2 = advect_scalar_grid(u0, s1), given g_s2 = dL/ds2."""
     _chk_mac(g, u0, "u0")
-    check(_lib.lib().fm_advect_scalar_grid_adj(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1),
+    check(_lib.lib().fm_advect_scalar_grid_adj(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), ptr(s1),
                                                ptr(g_s2), *_mac_opt(g, g_u0, "g_u0"), ptr(g_s1),
                                                stream_ptr(stream)), "fm_advect_scalar_grid_adj")
 
@@ -162,7 +176,7 @@ def advect_u_grid_adj(g: GridSpec, rk: int, dx: float, dt: float, u0, u1, g_u2, 
     """g_u0 += dL/du0 (backtrace), g_u1 += dL/du1 (sampled field) for u2 = advect_u_grid(u0, u1)."""
     for n, u in (("u0", u0), ("u1", u1), ("g_u2", g_u2)):
         _chk_mac(g, u, n)
-    check(_lib.lib().fm_advect_u_grid_adj(C.byref(g.c_grid()), _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
+    check(_lib.lib().fm_advect_u_grid_adj(g._ref, _dt(u0[0]), rk, dx, dt, *_mac3(u0), *_mac3(u1),
                                           *_mac3(g_u2), *_mac_opt(g, g_u0, "g_u0"), *_mac_opt(g, g_u1, "g_u1"),
                                           stream_ptr(stream)), "fm_advect_u_grid_adj")
 
@@ -172,7 +186,7 @@ def pullback_u_adj(g: GridSpec, dx: float, u0, T_f, psi_f, g_out, alpha=1.0, bet
     """Transpose of pullback_u: accumulates into g_u0, g_T, g_psi, g_base (any may be None)."""
     _chk_mac(g, u0, "u0")
     _chk_mac(g, g_out, "g_out")
-    check(_lib.lib().fm_pullback_u_adj(C.byref(g.c_grid()), _dt(u0[0]), dx, *_mac3(u0), *_mac3(T_f),
+    check(_lib.lib().fm_pullback_u_adj(g._ref, _dt(u0[0]), dx, *_mac3(u0), *_mac3(T_f),
                                        *_mac3(psi_f), alpha, beta, *_mac3(g_out), *_mac_opt(g, g_u0, "g_u0"),
                                        *_mac3(g_T), *_mac3(g_psi), *_mac_opt(g, g_base, "g_base"),
                                        stream_ptr(stream)), "fm_pullback_u_adj")
@@ -181,7 +195,7 @@ def pullback_u_adj(g: GridSpec, dx: float, u0, T_f, psi_f, g_out, alpha=1.0, bet
 def pullback_scalar_adj(g: GridSpec, dx: float, s0, psi, g_out, alpha=1.0, beta=0.0, g_s0=None, g_psi=None,
                         g_base=None, stream=None):
     """Transpose of pullback_scalar: accumulates into g_s0, g_psi, g_base (any may be None)."""
-    check(_lib.lib().fm_pullback_scalar_adj(C.byref(g.c_grid()), _dt(s0), dx, ptr(s0), ptr(psi), alpha, beta,
+    check(_lib.lib().fm_pullback_scalar_adj(g._ref, _dt(s0), dx, ptr(s0), ptr(psi), alpha, beta,
                                             ptr(g_out), ptr(g_s0), ptr(g_psi), ptr(g_base), stream_ptr(stream)),
           "fm_pullback_scalar_adj")
 
@@ -191,7 +205,7 @@ def rk_grid_adj(g: GridSpec, rk: int, dx: float, dt: float, face: int, psi, T, u
     """Transpose of rk_grid at its inputs (psi, T, u): accumulates into g_psi, g_T, g_u."""
     _chk_mac(g, u, "u")
     _chk_vec(g, psi, face, "psi")
-    check(_lib.lib().fm_rk_grid_adj(C.byref(g.c_grid()), _dt(psi), rk, dx, dt, face, ptr(psi), ptr(T), *_mac3(u),
+    check(_lib.lib().fm_rk_grid_adj(g._ref, _dt(psi), rk, dx, dt, face, ptr(psi), ptr(T), *_mac3(u),
                                     ptr(g_psi_out), ptr(g_T_out), ptr(g_psi), ptr(g_T), *_mac_opt(g, g_u, "g_u"),
                                     stream_ptr(stream)), "fm_rk_grid_adj")
 
@@ -201,7 +215,7 @@ def accumulate_init(g: GridSpec, dx: float, dt: float, f, init, F_f, phi_f, Hp=N
     hs = []
     for c in range(3):
         hs += [ptr(Hp[c]) if ab3 and c < g.dim else None, ptr(Hpp[c]) if ab3 and c < g.dim else None]
-    check(_lib.lib().fm_accumulate_init(C.byref(g.c_grid()), _dt(f[0]), dx, dt, int(ab3), ind, *_mac3(f),
+    check(_lib.lib().fm_accumulate_init(g._ref, _dt(f[0]), dx, dt, int(ab3), ind, *_mac3(f),
                                         *_mac3(init), *_mac3(F_f), *_mac3(phi_f), *hs, stream_ptr(stream)),
           "fm_accumulate_init")
 
@@ -214,7 +228,7 @@ def accumulate_init_pair(g: GridSpec, dx: float, dt: float, f, init, F_f, phi_f,
     hs = []
     for c in range(3):
         hs += [ptr(Hp[c]) if ab3 and c < g.dim else None, ptr(Hpp[c]) if ab3 and c < g.dim else None]
-    check(_lib.lib().fm_accumulate_init_pair(C.byref(g.c_grid()), _dt(f[0]), dx, dt, int(ab3), ind, *_mac3(f),
+    check(_lib.lib().fm_accumulate_init_pair(g._ref, _dt(f[0]), dx, dt, int(ab3), ind, *_mac3(f),
                                              *_mac3(init), *_mac3(F_f), *_mac3(phi_f), *hs, *_mac3(f2), dt2,
                                              stream_ptr(stream)), "fm_accumulate_init_pair")
 
@@ -222,18 +236,18 @@ def accumulate_init_pair(g: GridSpec, dx: float, dt: float, f, init, F_f, phi_f,
 def nabla_u_w(g: GridSpec, dx: float, u, w, r, order: Optional[int] = None, stream=None):
     if order is None:
         order = 3 if g.dim == 3 else 4
-    check(_lib.lib().fm_nabla_u_w(C.byref(g.c_grid()), _dt(u[0]), order, dx, *_mac3(u), *_mac3(w), *_mac3(r),
+    check(_lib.lib().fm_nabla_u_w(g._ref, _dt(u[0]), order, dx, *_mac3(u), *_mac3(w), *_mac3(r),
                                   stream_ptr(stream)), "fm_nabla_u_w")
 
 
 def nabla_scalar_adjoint(g: GridSpec, dx: float, s, adj, r, stream=None):
-    check(_lib.lib().fm_nabla_scalar_adjoint(C.byref(g.c_grid()), _dt(s), dx, ptr(s), ptr(adj), *_mac3(r),
+    check(_lib.lib().fm_nabla_scalar_adjoint(g._ref, _dt(s), dx, ptr(s), ptr(adj), *_mac3(r),
                                              stream_ptr(stream)), "fm_nabla_scalar_adjoint")
 
 
 def reset_to_identity(g: GridSpec, dx: float, psi_c, psi_f, T_f, stream=None):
     t = psi_c if psi_c is not None else (psi_f[0] if psi_f else T_f[0])
-    check(_lib.lib().fm_reset_to_identity(C.byref(g.c_grid()), _dt(t), dx, ptr(psi_c), *_mac3(psi_f), *_mac3(T_f),
+    check(_lib.lib().fm_reset_to_identity(g._ref, _dt(t), dx, ptr(psi_c), *_mac3(psi_f), *_mac3(T_f),
                                           stream_ptr(stream)), "fm_reset_to_identity")
 
 
@@ -260,7 +274,7 @@ def clamp_extrema(g: GridSpec, src, ref, dst, stream=None):
         raise _lib.FlowmapError(1, "clamp_extrema: src, ref and dst must share shape and dtype")
     if dst.data_ptr() == ref.data_ptr():
         raise _lib.FlowmapError(2, "clamp_extrema: dst may not alias ref")
-    check(_lib.lib().fm_clamp_extrema(C.byref(g.c_grid()), _dt(src), face, ptr(src), ptr(ref), ptr(dst),
+    check(_lib.lib().fm_clamp_extrema(g._ref, _dt(src), face, ptr(src), ptr(ref), ptr(dst),
                                       stream_ptr(stream)), "fm_clamp_extrema")
 
 
@@ -273,7 +287,7 @@ def store(src, dst, stream=None):
 
 
 def laplacian(g: GridSpec, p, Ap, stream=None):
-    check(_lib.lib().fm_laplacian(C.byref(g.c_grid()), _dt(p), ptr(p), ptr(Ap), stream_ptr(stream)), "fm_laplacian")
+    check(_lib.lib().fm_laplacian(g._ref, _dt(p), ptr(p), ptr(Ap), stream_ptr(stream)), "fm_laplacian")
 
 
 # ---------------------------------------------------------------------------
@@ -292,7 +306,7 @@ def vortex_velocity_2d(g: GridSpec, dx: float, theta, ux, uy, stream=None):
     """Faces of the point-vortex velocity of theta (split_central_vector of the centre values)."""
     _chk_mac(g, (ux, uy), "u")
     th, nv, tp = _theta_arg(theta)
-    check(_lib.lib().fm_vortex_velocity_2d(C.byref(g.c_grid()), _dt(ux), dx, nv, tp, ptr(ux), ptr(uy),
+    check(_lib.lib().fm_vortex_velocity_2d(g._ref, _dt(ux), dx, nv, tp, ptr(ux), ptr(uy),
                                            stream_ptr(stream)), "fm_vortex_velocity_2d")
 
 
@@ -301,7 +315,7 @@ def vortex_velocity_grad_2d(g: GridSpec, dx: float, theta, lam_x, lam_y, stream=
     th, nv, tp = _theta_arg(theta)
     work = torch.empty(592 * 3 * nv, dtype=torch.float64, device=lam_x.device)
     grad = torch.empty(3 * nv, dtype=torch.float64, device=lam_x.device)
-    check(_lib.lib().fm_vortex_velocity_grad_2d(C.byref(g.c_grid()), _dt(lam_x), dx, nv, tp, ptr(lam_x), ptr(lam_y),
+    check(_lib.lib().fm_vortex_velocity_grad_2d(g._ref, _dt(lam_x), dx, nv, tp, ptr(lam_x), ptr(lam_y),
                                                 ptr(work), ptr(grad), stream_ptr(stream)),
           "fm_vortex_velocity_grad_2d")
     return grad
@@ -309,14 +323,14 @@ def vortex_velocity_grad_2d(g: GridSpec, dx: float, theta, lam_x, lam_y, stream=
 
 def vorticity_2d(g: GridSpec, dx: float, ux, uy, omega, stream=None):
     _chk_mac(g, (ux, uy), "u")
-    check(_lib.lib().fm_vorticity_2d(C.byref(g.c_grid()), _dt(ux), dx, ptr(ux), ptr(uy), ptr(omega),
+    check(_lib.lib().fm_vorticity_2d(g._ref, _dt(ux), dx, ptr(ux), ptr(uy), ptr(omega),
                                      stream_ptr(stream)), "fm_vorticity_2d")
 
 
 def vorticity_loss_2d(g: GridSpec, dx: float, ux, uy, omega_target, lam_x, lam_y, work, part, loss, stream=None):
     """loss (device FP64, 1 entry) = sum (omega - omega*)^2; lam = (d omega/d u)^T 2 (omega - omega*)."""
     _chk_mac(g, (ux, uy), "u")
-    check(_lib.lib().fm_vorticity_loss_2d(C.byref(g.c_grid()), _dt(ux), dx, ptr(ux), ptr(uy), ptr(omega_target),
+    check(_lib.lib().fm_vorticity_loss_2d(g._ref, _dt(ux), dx, ptr(ux), ptr(uy), ptr(omega_target),
                                           ptr(work), ptr(part), ptr(lam_x), ptr(lam_y), ptr(loss), stream_ptr(stream)),
           "fm_vorticity_loss_2d")
 
@@ -337,7 +351,7 @@ def gaussian_force(g: GridSpec, dx: float, center, inv_radius, strength, f, stre
     reaching it (device parameter tensors: center n x dim, inv_radius n, strength n x dim)."""
     _chk_mac(g, f, "f")
     n = _chk_gaussians(g, center, inv_radius, strength, f[0].dtype)
-    check(_lib.lib().fm_gaussian_force(C.byref(g.c_grid()), _dt(f[0]), dx, n, ptr(center), ptr(inv_radius),
+    check(_lib.lib().fm_gaussian_force(g._ref, _dt(f[0]), dx, n, ptr(center), ptr(inv_radius),
                                        ptr(strength), *_mac3(f), stream_ptr(stream)), "fm_gaussian_force")
 
 
@@ -351,7 +365,7 @@ def gaussian_force_grad(g: GridSpec, dx: float, center, inv_radius, strength, ad
     for t in out:
         if t.dtype != torch.float64 or tuple(t.shape) != (n, g.dim):
             raise _lib.FlowmapError(1, "gaussian_force_grad outputs are FP64 n x dim")
-    check(_lib.lib().fm_gaussian_force_grad(C.byref(g.c_grid()), _dt(adj_u[0]), dx, n, ptr(center), ptr(inv_radius),
+    check(_lib.lib().fm_gaussian_force_grad(g._ref, _dt(adj_u[0]), dx, n, ptr(center), ptr(inv_radius),
                                             ptr(strength), *_mac3(adj_u), *[ptr(t) for t in out],
                                             stream_ptr(stream)), "fm_gaussian_force_grad")
     return out
@@ -366,7 +380,7 @@ def viscous_force_2d(g: GridSpec, nu: float, dx: float, u, vis, adj=None, part=N
     if adj is not None:
         _chk_mac(g, adj, "adj")
         a = [ptr(adj[0]), ptr(adj[1])]
-    check(_lib.lib().fm_viscous_force_2d(C.byref(g.c_grid()), _dt(u[0]), nu, dx, ptr(u[0]), ptr(u[1]), ptr(vis[0]),
+    check(_lib.lib().fm_viscous_force_2d(g._ref, _dt(u[0]), nu, dx, ptr(u[0]), ptr(u[1]), ptr(vis[0]),
                                          ptr(vis[1]), a[0], a[1], ptr(part), ptr(dot), stream_ptr(stream)),
           "fm_viscous_force_2d")
 
@@ -383,11 +397,11 @@ def mask_velocity(g: GridSpec, mask, u, bvel=None, stream=None):
     _chk_mac(g, u, "u")
     if bvel is not None:
         _chk_vec(g, bvel, -1, "bvel")
-    check(_lib.lib().fm_mask_velocity(C.byref(g.c_grid()), _dt(u[0]), _mask_arg(g, mask), ptr(bvel), *_mac3(u),
+    check(_lib.lib().fm_mask_velocity(g._ref, _dt(u[0]), _mask_arg(g, mask), ptr(bvel), *_mac3(u),
                                       stream_ptr(stream)), "fm_mask_velocity")
 
 
 def mask_passive(g: GridSpec, mask, s, adjoint: bool = False, stream=None):
     """mask_passive_by_boundary, or mask_adj_passive_by_boundary with adjoint=True."""
-    check(_lib.lib().fm_mask_passive(C.byref(g.c_grid()), _dt(s), _mask_arg(g, mask), ptr(s), int(adjoint),
+    check(_lib.lib().fm_mask_passive(g._ref, _dt(s), _mask_arg(g, mask), ptr(s), int(adjoint),
                                      stream_ptr(stream)), "fm_mask_passive")
