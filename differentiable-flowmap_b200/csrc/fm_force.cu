@@ -23,25 +23,27 @@
 // the Gaussian's separability, exp(-r s2) = exp(-r s2_other) exp(-r dz^2),
 // which differs from exp(-q) by a few ulps.
 //
-// B200 mapping.  3000 Gaussians against every face is compute work.  Both
-// kernels give each thread a column of faces along the fastest axis (k in 3D,
-// j in 2D), tabulate per Gaussian the squared offsets and the factors
-// exp(-r dx_a^2) in shared memory (every axis in the force kernel, the column
-// axis in the adjoint), and combine the other axes once per (column,
-// Gaussian); a face then costs two shared loads, a compare and an FMA.
-//  * k_gauss_force: one CTA per tile of cells (16x16 in 2D, 8x8x8 in 3D).  The
-//    CTA walks the Gaussians in chunks of 256 and appends those whose support
-//    ball (radius sqrt(5/r), widened) reaches the tile's box to a list in
-//    shared memory, in ascending order (ballot + popc prefix); once the list
-//    could not take another chunk, or at the end, it tabulates the listed
-//    Gaussians a sub-chunk at a time and every thread accumulates its column
-//    segment over them in list order.  The cull is a superset of the exact test.
-//  * k_gauss_grad: one CTA per Gaussian over the columns of its support box;
-//    each column's faces are summed in registers of the run's type and
-//    flushed to FP64 per column; fixed-order warp-shuffle + shared-memory
-//    reduction, so the result is deterministic (the reference's atomics are
-//    not).  Gaussians with r <= 0 or a support wider than the table take a
-//    per-face path in the reference's operation order.
+// B200 mapping.  3000 Gaussians against every face is compute work, bound by
+// issue slots.  Both kernels tabulate per Gaussian and axis the squared offsets and
+// the factors exp(-r dx_a^2) in shared memory, so that a face costs a few
+// additions, a compare and a multiply-add.
+//  * k_gauss_force: one CTA per tile of cells (16x16 in 2D, 8x8x8 in 3D), a
+//    column of faces along the fastest axis (k in 3D, j in 2D) per thread.  The
+//    CTA walks the Gaussians in chunks of 256, read one chunk ahead, and appends
+//    those whose support ball (radius sqrt(5/r), widened) reaches the tile's box
+//    to a list in shared memory, in ascending order (ballot + popc prefix); once
+//    the list could not take another chunk, or at the end, it tabulates the
+//    listed Gaussians a sub-chunk at a time (each thread its own table entry) and
+//    every thread accumulates its column segment over them in list order, the
+//    other axes combined once per (column, Gaussian), four faces per shared load.
+//    The cull is a superset of the exact test.  3000 Gaussians of radius 1..9 cells
+//    on 128^3 in FP32: 289 us with the cull in FP64 and scalar table loads, 210 us now.
+//  * k_gauss_grad: one CTA per Gaussian over its support; short stretches of
+//    faces are summed in registers of the run's type and flushed to FP64;
+//    fixed-order warp-shuffle + shared-memory reduction, so the result is
+//    deterministic (the reference's atomics are not).  Gaussians with r <= 0 or a
+//    support longer than the table along the columns take a per-face path in the
+//    reference's operation order.
 #include <math.h>
 
 #include "fm_common.cuh"
@@ -52,7 +54,8 @@ namespace fm {
 constexpr int kGfThreads = 256;
 constexpr int kGfWarps = kGfThreads / 32;
 constexpr int kGfMaxN = 1 << 24;
-constexpr int kGfTab = 256;   // column-table capacity of the adjoint kernel (faces)
+constexpr int kGfTab = 256;   // table capacity of the adjoint kernel (faces of an axis)
+constexpr int kGfFlush = 32;  // faces per lane after which its sums go to FP64
 
 // Tiles of the force kernel; the column axis is D-1.  SEG: faces per thread
 // along it (one segment per thread: 3D 9*8 + 8*9 + 8*8 = 208, 2D 17*4 + 16*5 = 148).
@@ -98,19 +101,31 @@ __device__ __forceinline__ bool gf_weight(const T* p, const T* c, T r, T* dp, T&
   return true;
 }
 
-// Tile cull: does Gaussian (c, r) possibly reach a face inside [lo, hi]?
+// Tile cull: does Gaussian (c, r) possibly reach a face inside [lo, hi]?  In the
+// run's type (every Gaussian is tested against every tile): the box is wider
+// than the faces by a hundredth of a cell and the bound by kGfMargin, far above the
+// rounding here, and s2 r is compared so that no division is needed.
 template <typename T, int D>
-__device__ __forceinline__ bool gf_touches(const T* c, T r, const double* lo, const double* hi) {
+__device__ __forceinline__ bool gf_touches(const T* c, T r, const T* lo, const T* hi) {
   if (r != r) return false;          // NaN radius: the exact test excludes every face
   if (!(r > (T)0)) return true;      // r <= 0: q <= 0 everywhere (left to the exact test)
-  double d2 = 0;
+  T d2 = (T)0;
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    const double x = (double)c[a];
-    const double t = x < lo[a] ? lo[a] - x : (x > hi[a] ? x - hi[a] : 0.0);
+    const T t = c[a] < lo[a] ? lo[a] - c[a] : (c[a] > hi[a] ? c[a] - hi[a] : (T)0);
     d2 += t * t;
   }
-  return d2 <= 5.0 / (double)r * (1.0 + kGfMargin);
+  return !(d2 * r > (T)(5.0 * (1.0 + kGfMargin)));  // NaN (0 times infinity, a NaN centre): left to the exact test
+}
+
+// four consecutive table entries, 16-byte aligned
+__device__ __forceinline__ void load4(const float* p, float* v) {
+  const float4 x = *reinterpret_cast<const float4*>(p);
+  v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+__device__ __forceinline__ void load4(const double* p, double* v) {
+  const double2 x = *reinterpret_cast<const double2*>(p), y = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
 }
 
 template <typename T, int D>
@@ -120,14 +135,15 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
                                                             T* __restrict__ f2) {
   using Tl = GfTile<D>;
   constexpr int CA = D - 1, SEG = Tl::SEG;
-  constexpr int BM = (Tl::B0 > Tl::BC ? Tl::B0 : Tl::BC) + 1;        // table entries per axis and variant
-  constexpr int SUB = sizeof(T) == 4 ? 64 : 32;                       // Gaussians tabulated at a time
+  // table entries per axis and variant, rounded up for 16-byte loads
+  constexpr int BM = ((Tl::B0 > Tl::BC ? Tl::B0 : Tl::BC) + 1 + 3) / 4 * 4;
+  constexpr int SUB = sizeof(T) == 4 ? 48 : 24;                       // Gaussians tabulated at a time
   constexpr int TS = D * 2 * BM;                                      // table entries per Gaussian
   constexpr int CAP = sizeof(T) == 4 ? 2 * kGfThreads : kGfThreads;  // culled-list capacity
   __shared__ T s_c[D][CAP], s_s[D][CAP], s_r[CAP];
   // per tabulated Gaussian l, axis a, variant v (0 cell, 1 face), index q - lo[a]:
   // squared offset and exp(-r offset^2)
-  __shared__ T t_sq[SUB][D][2][BM], t_ex[SUB][D][2][BM];
+  __shared__ alignas(16) T t_sq[SUB][D][2][BM], t_ex[SUB][D][2][BM];
   __shared__ T t_lo[SUB], t_hi[SUB];  // 5 (1 -+ m) / r, or +inf for r <= 0
   __shared__ int s_cnt[kGfWarps];
 
@@ -140,11 +156,11 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
   const int hc[3] = {min(lo[0] + Tl::B0, g.n[0]), min(lo[1] + Tl::B1, g.n[1]), min(lo[2] + Tl::B2, g.n[2])};
   // the tile's box: faces at i dx (the last tile along an axis also owns the
   // face at n dx), centres at (i + 1/2) dx, widened by a hundredth of a cell
-  double blo[3], bhi[3];
+  T blo[3], bhi[3];
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    blo[a] = ((double)lo[a] - 0.01) * (double)dx;
-    bhi[a] = ((double)hc[a] + 1.01) * (double)dx;
+    blo[a] = (T)(((double)lo[a] - 0.01) * (double)dx);
+    bhi[a] = (T)(((double)hc[a] + 1.01) * (double)dx);
   }
 
   // this thread's segment: component cc, tile-local other-axis indices io[],
@@ -179,25 +195,41 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
   }
   const int v0 = cc == 0 ? 1 : 0, v1 = cc == 1 ? 1 : 0, vc = cc == CA ? 1 : 0;
 
+  // the table entry this thread fills, for every (kGfThreads / TS)-th Gaussian: axis, variant, index
+  static_assert(TS <= kGfThreads, "one entry a thread");
+  const int te = threadIdx.x % TS, ta = te / (2 * BM), tv = te / BM % 2;
+  const int tq = threadIdx.x < kGfThreads / TS * TS ? te % BM : -1;
+  const T tpos = gf_pos<T>((ta == 0 ? lo[0] : (ta == 1 ? lo[1] : lo[2])) + tq, tv == 1, dx);
+
   T acc[SEG];
 #pragma unroll
   for (int m = 0; m < SEG; ++m) acc[m] = (T)0;
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int listed = 0;  // culled Gaussians waiting in the list (uniform across the CTA)
-  for (int base = 0; base < n; base += kGfThreads) {
-    const int I = base + threadIdx.x;
-    T c[D], s[D], r = (T)0;
-    bool hit = false;
+  T cn[D], rn = (T)NAN;  // the next chunk's Gaussian, read ahead (NaN: none)
+  const auto ahead = [&](int I) {
+    rn = (T)NAN;
     if (I < n) {
 #pragma unroll
-      for (int a = 0; a < D; ++a) {
-        c[a] = cen[(long)I * D + a];
-        s[a] = str[(long)I * D + a];
-      }
-      r = ir[I];
-      hit = gf_touches<T, D>(c, r, blo, bhi);
+      for (int a = 0; a < D; ++a) cn[a] = __ldg(cen + (long)I * D + a);
+      rn = __ldg(ir + I);
     }
+  };
+#pragma unroll
+  for (int a = 0; a < D; ++a) cn[a] = (T)0;
+  ahead(threadIdx.x);
+  for (int base = 0; base < n; base += kGfThreads) {
+    const int I = base + threadIdx.x;
+    T c[D], s[D];
+    const T r = rn;
+#pragma unroll
+    for (int a = 0; a < D; ++a) c[a] = cn[a];
+    ahead(I + kGfThreads);
+    const bool hit = gf_touches<T, D>(c, r, blo, bhi);
+    if (hit)
+#pragma unroll
+      for (int a = 0; a < D; ++a) s[a] = __ldg(str + (long)I * D + a);
     const unsigned m = __ballot_sync(0xffffffffu, hit);
     if (lane == 0) s_cnt[w] = __popc(m);
     __syncthreads();
@@ -225,19 +257,18 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
       listed = 0;
       for (int sub = 0; sub < tot; sub += SUB) {
         const int cnt = min(SUB, tot - sub);
-        for (int x = threadIdx.x; x < cnt * TS; x += kGfThreads) {
-          const int l = x / TS, rem = x - l * TS, a = rem / (2 * BM), rv = rem - a * 2 * BM, v = rv / BM,
-                    q = rv - v * BM;
-          const T rr = s_r[sub + l];
-          const T d = rn_sub(gf_pos<T>(lo[a] + q, v == 1, dx), s_c[a][sub + l]);
-          const T sq = rn_mul(d, d);
-          t_sq[l][a][v][q] = sq;
-          t_ex[l][a][v][q] = exp(-rn_mul(sq, rr));
-          if (rem == 0) {
-            const bool pos = rr > (T)0;
-            t_lo[l] = pos ? (T)(5.0 * (1.0 - kGfMargin)) / rr : (T)INFINITY;
-            t_hi[l] = pos ? (T)(5.0 * (1.0 + kGfMargin)) / rr : (T)INFINITY;
+        if (tq >= 0)
+          for (int l = threadIdx.x / TS; l < cnt; l += kGfThreads / TS) {
+            const T d = rn_sub(tpos, s_c[ta][sub + l]);
+            const T sq = rn_mul(d, d);
+            t_sq[l][ta][tv][tq] = sq;
+            t_ex[l][ta][tv][tq] = exp(-rn_mul(sq, s_r[sub + l]));
           }
+        if (threadIdx.x < cnt) {
+          const T rr = s_r[sub + threadIdx.x];
+          const bool pos = rr > (T)0;
+          t_lo[threadIdx.x] = pos ? (T)(5.0 * (1.0 - kGfMargin)) / rr : (T)INFINITY;
+          t_hi[threadIdx.x] = pos ? (T)(5.0 * (1.0 + kGfMargin)) / rr : (T)INFINITY;
         }
         __syncthreads();
         if (cc >= 0) {
@@ -253,17 +284,32 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
             if (B < (T)0) continue;  // the column misses the support
             const T A = t_lo[l] - sxy, rr = s_r[sub + l];
             const T ev = exy * s_s[cc][sub + l];
+            // entries past the segment's end are only added to sums that are not stored
+            const T* const psq = &t_sq[l][CA][vc][k0];
+            const T* const pex = &t_ex[l][CA][vc][k0];
+            T sq[SEG];
+            bool near = false;
 #pragma unroll
-            for (int q = 0; q < SEG; ++q) {
-              if (q < len) {
-                const T sq = t_sq[l][CA][vc][k0 + q];
-                bool in = sq < A;
-                if (!in && sq <= B) {
-                  const T d = sqrt(rn_add(sxy, sq));
-                  in = rn_mul(rn_mul(d, d), rr) < (T)5;
-                }
-                if (in) acc[q] += ev * t_ex[l][CA][vc][k0 + q];
+            for (int q0 = 0; q0 < SEG; q0 += 4) {
+              if (q0 + 4 > SEG && len <= q0) break;  // 3D: the ninth face, in the last tiles only
+              T x4[4], e4[4];
+              load4(psq + q0, x4);
+              load4(pex + q0, e4);
+#pragma unroll
+              for (int q = q0; q < SEG && q < q0 + 4; ++q) {
+                sq[q] = x4[q - q0];
+                const bool in = sq[q] < A;
+                if (in) acc[q] += ev * e4[q - q0];
+                near |= !in & (sq[q] <= B);
               }
+            }
+            if (near) {  // rare
+#pragma unroll
+              for (int q = 0; q < SEG; ++q)
+                if (q < len && !(sq[q] < A) && sq[q] <= B) {
+                  const T d = sqrt(rn_add(sxy, sq[q]));
+                  if (rn_mul(rn_mul(d, d), rr) < (T)5) acc[q] += ev * pex[q];
+                }
             }
           }
         }
@@ -283,19 +329,11 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
   }
 }
 
-// Face-index range along axis `a` of component-`c` faces within the support
-// of a Gaussian at x with widened radius R (R < 0: the whole axis).
-__device__ __forceinline__ void gf_axis_range(double x, double R, double dx, bool face_axis, int len, int& i0,
-                                              int& i1) {
-  if (R < 0) {
-    i0 = 0;
-    i1 = len - 1;
-    return;
-  }
+// Face-index range along one axis within [lo, hi] (in cells; the bounds are
+// widened by a hundredth of a cell, far above their rounding).
+__device__ __forceinline__ void gf_axis_range(double lo, double hi, bool face_axis, int len, int& i0, int& i1) {
   const double off = face_axis ? 0.0 : 0.5;
-  double a = ceil((x - R) / dx - off) - 1.0, b = floor((x + R) / dx - off) + 1.0;
-  a = fmax(a, 0.0);
-  b = fmin(b, (double)(len - 1));
+  const double a = fmax(ceil(lo - off), 0.0), b = fmin(floor(hi - off), (double)(len - 1));
   if (!(a <= b)) {
     i0 = 1;
     i1 = 0;
@@ -305,20 +343,115 @@ __device__ __forceinline__ void gf_axis_range(double x, double R, double dx, boo
   i1 = (int)b;
 }
 
+// Offset, its square and exp(-r offset^2) of one face index along an axis.
+template <typename T> struct alignas(4 * sizeof(T)) GfAxis {
+  T dp, sq, ex, pad;
+};
+template <typename T>
+__device__ __forceinline__ GfAxis<T> gf_axis(int i, bool face, T dx, T c, T r) {
+  const T d = rn_sub(gf_pos<T>(i, face, dx), c), sq = rn_mul(d, d);
+  return {d, sq, exp(-rn_mul(sq, r)), (T)0};
+}
+
+// One warp's piece of a support in the adjoint kernel: 8 faces of the column
+// axis from q0 on, at one index of the outer axis (offset d0, its square, its
+// factor), times the middle-axis indices ma..mb of the slab.
+template <typename T> struct alignas(16) GfTask {
+  const T* row;     // the first of the 8 faces, at the slab's start
+  unsigned rowst;   // a step along the middle axis
+  short q0, last;   // last: of the 8 faces within the range
+  short ma, mb, mlast, cc;
+  T d0, sq0, ex0;
+};
+
+// The Gaussian that block b takes: a one-to-one map that puts wide supports
+// first, in four classes of radius, so that the last blocks to run are short ones
+// (a support of 20 cells is 60 times the work of one of 5).  Every block
+// counts the classes for itself: worth it while that is a few loads a thread;
+// far more blocks than fit at once even out by themselves.
+constexpr int kGfOrderMax = 32 * kGfThreads;
+template <typename T>
+__device__ __forceinline__ int gf_order(int b, int n, const T* __restrict__ ir) {
+  __shared__ T s_min[kGfWarps];
+  __shared__ unsigned long long s_cnt[kGfWarps];
+  __shared__ int s_pick;
+  if (n > kGfOrderMax) return b;
+  constexpr unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T least = (T)INFINITY;
+  for (int i = threadIdx.x; i < n; i += kGfThreads) {
+    const T r = __ldg(ir + i);
+    if (r > (T)0) least = min(least, r);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) least = min(least, __shfl_xor_sync(all, least, o));
+  if (lane == 0) s_min[w] = least;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kGfWarps; ++k) least = min(least, s_min[k]);
+  // radii above 3/4, 1/2, 1/4 of the widest; r <= 0 (every face) with the widest, NaN with the narrowest
+  const auto bin = [&](T r) { return (r <= least * (T)1.78 ? 0 : (r <= least * (T)4 ? 1 : (r <= least * (T)16 ? 2 : 3))); };
+  unsigned packed = 0;  // four counts of at most 32
+  for (int i = threadIdx.x; i < n; i += kGfThreads) packed += 1u << (8 * bin(__ldg(ir + i)));
+  unsigned long long mine = 0;  // ... in 16 bits each, for the sums over the block
+#pragma unroll
+  for (int k = 0; k < 4; ++k) mine |= (unsigned long long)(packed >> (8 * k) & 0xff) << (16 * k);
+  unsigned long long upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long x = __shfl_up_sync(all, upto, o);
+    if (lane >= o) upto += x;
+  }
+  if (lane == 31) s_cnt[w] = upto;
+  __syncthreads();
+  unsigned long long total = 0;
+#pragma unroll
+  for (int k = 0; k < kGfWarps; ++k) {
+    if (k < w) upto += s_cnt[k];
+    total += s_cnt[k];
+  }
+  int k = 0, p = b;  // block b is the p-th of class k
+  while (k < 3 && p >= (int)(total >> (16 * k) & 0xffff)) p -= (int)(total >> (16 * k++) & 0xffff);
+  p -= (int)((upto - mine) >> (16 * k) & 0xffff);
+  if (p >= 0 && p < (int)(mine >> (16 * k) & 0xffff))
+    for (int i = threadIdx.x; i < n; i += kGfThreads)
+      if (bin(__ldg(ir + i)) == k && p-- == 0) s_pick = i;
+  __syncthreads();
+  return s_pick;
+}
+
 // Per-Gaussian sums v[c] adj_strength, v[D+a] adj_center, v[2D+c]
 // pen_strength, v[3D+a] pen_center (FP64).
+//
+// Bound by issue slots: about 19 instructions a face, plus what is done per warp
+// and not per face.  So the support, a ball, is split to waste few lanes, and
+// what a whole warp would compute alike is computed by one thread each.  A task
+// is 8 faces of the column axis (k in 3D, j in 2D; contiguous in memory) at one
+// index of the outer axis; its warp walks, 4 faces at a time, the stretch of the
+// middle axis that the ball reaches there.  Every thread prepares one task, then
+// the warps take them in turn.  The column's factors stay in registers, the
+// middle axis' come from shared memory.  Sums of the run's type are flushed to
+// FP64 once they hold kGfFlush faces.  3000 Gaussians of radius 1..9 cells on 128^3
+// in FP32: 334 us with a lane per column (strided loads, 32 unequal columns per
+// warp) and 206 us now.
 template <typename T, int D>
-__global__ void __launch_bounds__(kGfThreads, 4) k_gauss_grad(fm_grid g, T dx, const T* __restrict__ cen,
-                                                              const T* __restrict__ ir, const T* __restrict__ str,
-                                                              const T* __restrict__ a0, const T* __restrict__ a1,
-                                                              const T* __restrict__ a2, double* __restrict__ adj_c,
-                                                              double* __restrict__ adj_s, double* __restrict__ pen_c,
-                                                              double* __restrict__ pen_s) {
+__global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
+    k_gauss_grad(fm_grid g, T dx, int n, const T* __restrict__ cen, const T* __restrict__ ir, const T* __restrict__ str,
+                 const T* __restrict__ a0, const T* __restrict__ a1, const T* __restrict__ a2,
+                 double* __restrict__ adj_c, double* __restrict__ adj_s, double* __restrict__ pen_c,
+                 double* __restrict__ pen_s) {
   constexpr int NV = 4 * D;
-  constexpr int CA = D - 1;
+  constexpr int CA = D - 1, MA = D - 2;  // column and middle axis
+  constexpr int LC = 8, LM = 32 / LC, UN = 2, PAD = LM * UN;
+  constexpr int kStretch = 32;           // 2D has no outer axis: middle stretches instead
+  static_assert(kStretch % PAD == 0 && kGfTab % kStretch == 0, "stretches end where a step ends");
   __shared__ double s_red[kGfWarps][NV];
-  __shared__ T t_dp[kGfTab], t_ex[kGfTab];
-  const int I = blockIdx.x;
+  // by variant v (0 cells, 1 faces) of the axis; t_mid is one slab of the axis
+  __shared__ GfAxis<T> t_col[2][kGfTab], t_mid[2][kGfTab + PAD];
+  __shared__ GfTask<T> s_task[kGfThreads];
+  __shared__ int s_i0[D][2], s_len[D][2];  // the support's index range along an axis
+  const int I = gf_order<T>(blockIdx.x, n, ir);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   T c[D], s[D];
 #pragma unroll
   for (int a = 0; a < D; ++a) {
@@ -326,119 +459,198 @@ __global__ void __launch_bounds__(kGfThreads, 4) k_gauss_grad(fm_grid g, T dx, c
     s[a] = str[(long)I * D + a];
   }
   const T r = ir[I];
-  // support radius (widened) or -1 for "every face"; NaN r or a non-finite
-  // centre with r > 0 reaches no face
-  double R = -1.0;
-  bool none = r != r;
-  if (r > (T)0) {
-    R = sqrt(5.0 / (double)r) * (1.0 + kGfMargin) + 0.01 * (double)dx;
+  // NaN or infinite r, or a non-finite centre with r > 0, reaches no face; r <= 0 every face
+  bool none = r != r || r == (T)INFINITY;
+  if (r > (T)0)
 #pragma unroll
     for (int a = 0; a < D; ++a) none = none || !isfinite((double)c[a]);
+  if (threadIdx.x < 2 * D) {
+    const int a = threadIdx.x >> 1, v = threadIdx.x & 1;
+    double lo = -1.0, hi = 1e9;
+    if (r > (T)0) {
+      const double R = sqrt(5.0 / (double)r) * (1.0 + kGfMargin) + 0.01 * (double)dx;
+      const double x = (double)(a == 0 ? c[0] : (a == 1 ? c[1] : c[CA]));
+      lo = (x - R) / (double)dx;
+      hi = (x + R) / (double)dx;
+    }
+    int b0 = 1, b1 = 0;
+    if (!none) gf_axis_range(lo, hi, v == 1, (a == 0 ? g.n[0] : (a == 1 ? g.n[1] : g.n[2])) + v, b0, b1);
+    s_i0[a][v] = b0;
+    s_len[a][v] = b1 - b0 + 1;
   }
+  __syncthreads();
   double v[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = 0.0;
 
+  const T tlo = (T)(5.0 * (1.0 - kGfMargin)) / r, thi = (T)(5.0 * (1.0 + kGfMargin)) / r;
+  const T inv = (T)1 / dx;
+  // component cc's range; `cols`: its columns fit the table, and there is a ball
+  const auto start = [&](int cc, int a) { return s_i0[a][cc == a]; };
+  const auto extent = [&](int cc, int a) { return s_len[a][cc == a]; };
+  const auto cols = [&](int cc) { return r > (T)0 && extent(cc, CA) <= kGfTab; };
+  const int mlen = max(s_len[MA][0], s_len[MA][1]);
+  T S = (T)0, S0 = (T)0, Sm = (T)0, Sc = (T)0, E = (T)0, E0 = (T)0, Em = (T)0, Ec = (T)0;
+  int held = 0, hc = 0;  // faces per lane in these sums, and their component
+  const auto flush = [&]() {
+    T sc = s[0];
+#pragma unroll
+    for (int cc = 0; cc < D; ++cc)
+      if (hc == cc) {
+        sc = s[cc];
+        v[cc] += (double)S;
+        v[2 * D + cc] += 2.0 * (double)sc * (double)E;
+      }
+    const double k1 = 2.0 * (double)sc * (double)r, k2 = 2.0 * (double)sc * k1;
+    if (D == 3) v[D] += k1 * (double)S0, v[3 * D] += k2 * (double)E0;
+    v[D + MA] += k1 * (double)Sm, v[3 * D + MA] += k2 * (double)Em;
+    v[D + CA] += k1 * (double)Sc, v[3 * D + CA] += k2 * (double)Ec;
+    S = S0 = Sm = Sc = E = E0 = Em = Ec = (T)0;
+    held = 0;
+  };
+  for (int m0 = 0; m0 < mlen && r > (T)0; m0 += kGfTab) {  // the middle axis in slabs of the table's length
+    if (m0 > 0) __syncthreads();
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (m0 == 0)
+        for (int q = threadIdx.x; q < min(s_len[CA][f], kGfTab); q += kGfThreads)
+          t_col[f][q] = gf_axis<T>(s_i0[CA][f] + q, f == 1, dx, c[CA], r);
+      const int ms = min(kGfTab, s_len[MA][f] - m0);
+      for (int q = threadIdx.x; q < ms + PAD; q += kGfThreads)
+        t_mid[f][q] = q < ms ? gf_axis<T>(s_i0[MA][f] + m0 + q, f == 1, dx, c[MA], r)
+                             : GfAxis<T>{(T)0, (T)INFINITY, (T)0, (T)0};  // past the end: outside
+    }
+    int first[D + 1] = {0};  // each component's first task
+#pragma unroll
+    for (int cc = 0; cc < D; ++cc) {
+      const int ms = min(kGfTab, extent(cc, MA) - m0);
+      const int nout = D == 3 ? extent(cc, 0) : (ms + kStretch - 1) / kStretch;
+      const bool any = ms > 0 && nout > 0 && cols(cc);
+      first[cc + 1] = first[cc] + (any ? (extent(cc, CA) + LC - 1) / LC * nout : 0);
+    }
+    for (int tb = 0; tb < first[D]; tb += kGfThreads) {
+      const int t = tb + threadIdx.x;
+      if (t < first[D]) {
+        const int cc = t < first[1] ? 0 : (D == 2 || t < first[2] ? 1 : 2);
+        const int tt = t - (cc == 0 ? 0 : (cc == 1 ? first[1] : first[2 < D ? 2 : 1]));
+        const int ecol = extent(cc, CA), ms = min(kGfTab, extent(cc, MA) - m0);
+        const int chunks = (ecol + LC - 1) / LC, o = tt / chunks, q0 = (tt - o * chunks) * LC;
+        GfAxis<T> out = {(T)0, (T)0, (T)1, (T)0};
+        if (D == 3) out = gf_axis<T>(start(cc, 0) + o, cc == 0, dx, c[0], r);
+        // the stretch that the ball reaches at the chunk's nearest face, widened
+        // to whole indices; the centre in the slab's indices
+        const T za = rn_sub(gf_pos<T>(start(cc, CA) + q0, cc == CA, dx), c[CA]);
+        const T zb = rn_sub(gf_pos<T>(start(cc, CA) + min(q0 + LC, ecol) - 1, cc == CA, dx), c[CA]);
+        const T zm = za > (T)0 ? za : (zb < (T)0 ? zb : (T)0);
+        const T rest = thi - out.sq - zm * zm;
+        const T half = sqrt(rest) * inv + (T)0.01;
+        const T cm = -rn_sub(gf_pos<T>(start(cc, MA) + m0, cc == MA, dx), c[MA]) * inv;
+        const T mlo = D == 3 ? (T)0 : (T)(o * kStretch);
+        const T mhi = D == 3 ? (T)(ms - 1) : (T)min(ms - 1, o * kStretch + kStretch - 1);
+        int ma = 0, mb = -1;
+        if (rest >= (T)0) {  // false for NaN
+          ma = (int)min(max(floor(cm - half), mlo), mhi + (T)1);
+          mb = (int)max(min(ceil(cm + half), mhi), (T)-1);
+          if (D == 2) ma &= ~(PAD - 1);  // so that the last step stays within the stretch
+        }
+        const Shape fs = face_shape(g, cc);
+        GfTask<T> k;
+        k.row = (cc == 0 ? a0 : (cc == 1 ? a1 : a2)) +
+                (D == 3 ? fs.idx(start(cc, 0) + o, start(cc, 1) + m0, start(cc, CA) + q0)
+                        : fs.idx(start(cc, 0) + m0, start(cc, 1) + q0, 0));
+        k.rowst = D == 3 ? fs.s2 : fs.s1;
+        k.q0 = (short)q0, k.last = (short)(min(q0 + LC, ecol) - 1 - q0), k.cc = (short)cc;
+        k.ma = (short)ma, k.mb = (short)mb, k.mlast = (short)(ms - 1);
+        k.d0 = out.dp, k.sq0 = out.sq, k.ex0 = out.ex;
+        s_task[threadIdx.x] = k;
+      }
+      __syncthreads();
+      for (int t = w; t < min(kGfThreads, first[D] - tb); t += kGfWarps) {
+        const GfTask<T> k = s_task[t];
+        if (k.ma > k.mb) continue;
+        const int cc = k.cc;
+        if (held >= kGfFlush || (cc != hc && held > 0)) flush();
+        hc = cc;
+        held += (k.mb - k.ma) / LM + UN;
+        const int lc = min(lane & (LC - 1), (int)k.last);
+        const GfAxis<T> col = t_col[cc == CA][k.q0 + lc];
+        const T zsq = lc == (lane & (LC - 1)) ? col.sq : (T)INFINITY;  // past the end: outside
+        const T eoc = k.ex0 * col.ex;
+        const T* row = k.row + lc;
+        const int mlast = k.mlast;
+        const unsigned rowst = k.rowst;
+        const GfAxis<T>* const mid = t_mid[cc == MA];
+        T P = (T)0, Q = (T)0;
+        for (int m = k.ma + lane / LC; m - lane / LC <= k.mb; m += PAD) {
+          T av[UN], s2[UN], e[UN], dm[UN];
+          bool in[UN], near = false;
+#pragma unroll
+          for (int h = 0; h < UN; ++h) av[h] = __ldg(row + (unsigned)min(m + h * LM, mlast) * rowst);
+#pragma unroll
+          for (int h = 0; h < UN; ++h) {
+            const GfAxis<T> x = mid[m + h * LM];
+            dm[h] = x.dp;
+            e[h] = eoc * x.ex;
+            // s2 < tlo: inside off the boundary; s2 > thi: outside; between: the exact test
+            s2[h] = rn_add(D == 3 ? rn_add(k.sq0, x.sq) : x.sq, zsq);
+            in[h] = s2[h] < tlo;
+            near |= !in[h] & (s2[h] <= thi);
+          }
+          if (near) {  // rare
+#pragma unroll
+            for (int h = 0; h < UN; ++h)
+              if (!in[h] && s2[h] <= thi) {
+                const T d = sqrt(s2[h]);
+                in[h] = rn_mul(rn_mul(d, d), r) < (T)5;
+              }
+          }
+#pragma unroll
+          for (int h = 0; h < UN; ++h) {  // selects: a NaN outside stays out
+            const T ea = in[h] ? e[h] * av[h] : (T)0, e2 = in[h] ? e[h] * e[h] : (T)0;
+            P += ea;
+            Sm += ea * dm[h];
+            Q += e2;
+            Em += e2 * dm[h];
+          }
+        }
+        S += P, Sc += col.dp * P;
+        E += Q, Ec += col.dp * Q;
+        if (D == 3) S0 += k.d0 * P, E0 += k.d0 * Q;
+      }
+      __syncthreads();  // the tasks' last readers are done
+    }
+  }
+  if (held > 0) flush();
   if (!none) {
 #pragma unroll
     for (int cc = 0; cc < D; ++cc) {
+      const int e0 = extent(cc, 0), e1 = extent(cc, 1), e2 = D == 3 ? extent(cc, CA) : 1;
+      if (cols(cc) || e0 <= 0 || e1 <= 0 || e2 <= 0) continue;
+      // per-face path (r <= 0, or a support wider than the table), in the
+      // reference's operation order per face
       const Shape fs = face_shape(g, cc);
       const T* const adj = cc == 0 ? a0 : (cc == 1 ? a1 : a2);
-      int i0[3] = {0, 0, 0}, i1[3] = {0, 0, 0};
-#pragma unroll
-      for (int a = 0; a < D; ++a) gf_axis_range((double)c[a], R, (double)dx, a == cc, axis_len(fs, a), i0[a], i1[a]);
-      const int e0 = i1[0] - i0[0] + 1, e1 = i1[1] - i0[1] + 1, e2 = i1[2] - i0[2] + 1;
-      if (e0 <= 0 || e1 <= 0 || e2 <= 0) continue;
-      const int ecol = CA == 2 ? e2 : e1;
+      const int i0[3] = {start(cc, 0), start(cc, 1), D == 3 ? start(cc, CA) : 0};
       const T sc = s[cc];
-      if (r > (T)0 && ecol <= kGfTab) {
-        // column path: the column axis tabulated, the other axes per column
-        __syncthreads();  // the previous component's columns are done with the table
-        for (int q = threadIdx.x; q < ecol; q += kGfThreads) {
-          const T dz = rn_sub(gf_pos<T>(i0[CA] + q, cc == CA, dx), c[CA]);
-          t_dp[q] = dz;
-          t_ex[q] = exp(-rn_mul(rn_mul(dz, dz), r));
-        }
-        __syncthreads();
-        const double k1 = 2.0 * (double)sc * (double)r, k2 = 4.0 * (double)sc * (double)sc * (double)r,
-                     k3 = 2.0 * (double)sc;
-        const double rcap = 5.0 * (1.0 + kGfMargin) / (double)r, off = cc == CA ? 0.0 : 0.5;
-        const T tlo = (T)(5.0 * (1.0 - kGfMargin)) / r, thi = (T)(5.0 * (1.0 + kGfMargin)) / r;
-        const int ncol = D == 3 ? e0 * e1 : e0;
-        for (int col = threadIdx.x; col < ncol; col += kGfThreads) {
-          int io[2] = {0, 0};
-          if (D == 3) {
-            io[0] = i0[0] + col / e1;
-            io[1] = i0[1] + col % e1;
-          } else {
-            io[0] = i0[0] + col;
-          }
-          T dpo[2] = {(T)0, (T)0}, sxy = (T)0;
+      const unsigned cnt = (unsigned)e0 * (unsigned)e1 * (unsigned)e2;  // < 2^32 (validate_grid)
+      for (unsigned q = threadIdx.x; q < cnt; q += kGfThreads) {
+        const unsigned ij = q / (unsigned)e2;
+        const int k = (int)(q - ij * (unsigned)e2);
+        const unsigned ii = ij / (unsigned)e1;
+        const int j = (int)(ij - ii * (unsigned)e1), i = (int)ii;
+        T p[D], dp[D], e;
+        node_pos<T, D>(cc, i0[0] + i, i0[1] + j, i0[2] + k, dx, p);
+        if (!gf_weight<T, D>(p, c, r, dp, e)) continue;
+        const T av = adj[fs.idx(i0[0] + i, i0[1] + j, i0[2] + k)];
+        const T f = rn_mul(e, sc);
+        v[cc] += (double)rn_mul(e, av);
+        v[2 * D + cc] += (double)rn_mul(rn_mul((T)2, f), e);
+        const T ga = rn_mul(rn_mul(sc, e), (T)2);
+        const T gp = rn_mul(rn_mul(rn_mul(rn_mul((T)2, f), sc), e), (T)2);
 #pragma unroll
-          for (int a = 0; a < CA; ++a) {
-            dpo[a] = rn_sub(gf_pos<T>(io[a], a == cc, dx), c[a]);
-            sxy = a == 0 ? rn_mul(dpo[a], dpo[a]) : rn_add(sxy, rn_mul(dpo[a], dpo[a]));
-          }
-          // dz^2 < A: inside off the boundary; dz^2 > B: outside; between: the exact test
-          const T A = tlo - sxy, B = thi - sxy;
-          if (B < (T)0) continue;  // the column misses the support
-          // the column's included faces lie within |dz| <= sqrt(5 (1 + m) / r - sxy)
-          const double half = sqrt(fmax(rcap - (double)sxy, 0.0)) + 0.01 * (double)dx;
-          const int qa = max(0, (int)ceil(((double)c[CA] - half) / (double)dx - off) - 1 - i0[CA]);
-          const int qb = min(ecol - 1, (int)floor(((double)c[CA] + half) / (double)dx - off) + 1 - i0[CA]);
-          const T exy = exp(-rn_mul(sxy, r));
-          // the column axis is contiguous in memory (3D: k; 2D: j, where s2 == 1)
-          const T* row = adj + (D == 3 ? fs.idx(io[0], io[1], i0[2]) : fs.idx(io[0], i0[1], 0));
-          T sea = (T)0, seaz = (T)0, se2 = (T)0, se2z = (T)0;
-          // straight-line body (weights selected to 0 outside): the loads pipeline
-#pragma unroll 4
-          for (int q = qa; q <= qb; ++q) {
-            const T dz = t_dp[q], sq = rn_mul(dz, dz);
-            bool in = sq < A;
-            if (!in && sq <= B) {  // rare: a face within the margin of the cutoff
-              const T d = sqrt(rn_add(sxy, sq));
-              in = rn_mul(rn_mul(d, d), r) < (T)5;
-            }
-            const T e = exy * t_ex[q], av = __ldg(row + q);
-            const T ea = in ? e * av : (T)0, e2 = in ? e * e : (T)0;  // selects: a NaN outside stays out
-            sea += ea;
-            seaz += ea * dz;
-            se2 += e2;
-            se2z += e2 * dz;
-          }
-          v[cc] += (double)sea;
-          v[2 * D + cc] += k3 * (double)se2;
-#pragma unroll
-          for (int a = 0; a < CA; ++a) {
-            v[D + a] += k1 * (double)dpo[a] * (double)sea;
-            v[3 * D + a] += k2 * (double)dpo[a] * (double)se2;
-          }
-          v[D + CA] += k1 * (double)seaz;
-          v[3 * D + CA] += k2 * (double)se2z;
-        }
-      } else {
-        // per-face path (r <= 0, or a support wider than the table), in the
-        // reference's operation order per face
-        const unsigned cnt = (unsigned)e0 * (unsigned)e1 * (unsigned)e2;  // < 2^32 (validate_grid)
-        for (unsigned q = threadIdx.x; q < cnt; q += kGfThreads) {
-          const unsigned ij = q / (unsigned)e2;
-          const int k = (int)(q - ij * (unsigned)e2);
-          const unsigned ii = ij / (unsigned)e1;
-          const int j = (int)(ij - ii * (unsigned)e1), i = (int)ii;
-          T p[D], dp[D], e;
-          node_pos<T, D>(cc, i0[0] + i, i0[1] + j, i0[2] + k, dx, p);
-          if (!gf_weight<T, D>(p, c, r, dp, e)) continue;
-          const T av = adj[fs.idx(i0[0] + i, i0[1] + j, i0[2] + k)];
-          const T f = rn_mul(e, sc);
-          v[cc] += (double)rn_mul(e, av);
-          v[2 * D + cc] += (double)rn_mul(rn_mul((T)2, f), e);
-          const T ga = rn_mul(rn_mul(sc, e), (T)2);
-          const T gp = rn_mul(rn_mul(rn_mul(rn_mul((T)2, f), sc), e), (T)2);
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-            v[D + a] += (double)rn_mul(rn_mul(rn_mul(ga, dp[a]), r), av);
-            v[3 * D + a] += (double)rn_mul(rn_mul(gp, dp[a]), r);
-          }
+        for (int a = 0; a < D; ++a) {
+          v[D + a] += (double)rn_mul(rn_mul(rn_mul(ga, dp[a]), r), av);
+          v[3 * D + a] += (double)rn_mul(rn_mul(gp, dp[a]), r);
         }
       }
     }
@@ -451,7 +663,6 @@ __global__ void __launch_bounds__(kGfThreads, 4) k_gauss_grad(fm_grid g, T dx, c
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     v[k] = x;
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0)
 #pragma unroll
     for (int k = 0; k < NV; ++k) s_red[w][k] = v[k];
@@ -491,10 +702,10 @@ int gauss_grad(const fm_grid& g, double dx, int n, const void* cen, const void* 
                cudaStream_t s) {
   if (n == 0) return FM_OK;
   if (g.dim == 2)
-    launch(k_gauss_grad<T, 2>, (unsigned)n, kGfThreads, 0, s, g, (T)dx, (const T*)cen, (const T*)ir, (const T*)str,
+    launch(k_gauss_grad<T, 2>, (unsigned)n, kGfThreads, 0, s, g, (T)dx, n, (const T*)cen, (const T*)ir, (const T*)str,
            (const T*)ax, (const T*)ay, (const T*)nullptr, adj_c, adj_s, pen_c, pen_s);
   else
-    launch(k_gauss_grad<T, 3>, (unsigned)n, kGfThreads, 0, s, g, (T)dx, (const T*)cen, (const T*)ir, (const T*)str,
+    launch(k_gauss_grad<T, 3>, (unsigned)n, kGfThreads, 0, s, g, (T)dx, n, (const T*)cen, (const T*)ir, (const T*)str,
            (const T*)ax, (const T*)ay, (const T*)az, adj_c, adj_s, pen_c, pen_s);
   return check_cuda();
 }
