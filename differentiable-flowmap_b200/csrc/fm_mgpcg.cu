@@ -148,6 +148,30 @@ __device__ __forceinline__ void block_reduce2(double a, double b, double* out2) 
   }
 }
 
+// the same for a block of 32 x n threads (its partial sums in the same place)
+__device__ __forceinline__ void block_reduce2_2d(double a, double b, double* out2) {
+  __shared__ double sa[32], sb[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (threadIdx.x == 0) { sa[threadIdx.y] = a; sb[threadIdx.y] = b; }
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    a = b = 0.0;
+    for (unsigned k = 0; k < blockDim.y; ++k) a += sa[k], b += sb[k];
+    out2[0] = a;
+    out2[1] = b;
+  }
+}
+// a grid of fewer blocks than partial sums: the rest is zero
+__device__ __forceinline__ void walk_clear(double* part) {
+  if (blockIdx.x == 0)
+    for (unsigned q = gridDim.x + threadIdx.y * blockDim.x + threadIdx.x; q < kRedBlocks; q += blockDim.x * blockDim.y)
+      part[2 * q] = part[2 * q + 1] = 0.0;
+}
+
 // Sum the fixed-grid partials in a fixed order (one CTA of 256 threads).
 __device__ __forceinline__ void sum_partials(const double* __restrict__ part, double& a, double& b) {
   double x = 0, y = 0;
@@ -417,23 +441,6 @@ __global__ void k_dc_update_g(long n, double* __restrict__ x, const float* __res
   FM_GRID_STRIDE(q, n) x[q] += sc * (double)e[q];
 }
 
-// u -= grad x in FP64, rounded to FP32 (apply_bc: wall faces zero)
-template <int D>
-__global__ void k_dc_subgrad(fm_grid g, const double* __restrict__ x, MacW<float> u) {
-  pdl_begin();
-  const int c = blockIdx.y;
-  const Shape fs = face_shape(g, c);
-  const Shape cs = cell_shape(g);
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= fs.size()) return;
-  int I[3];
-  unflatten(fs, q, I[0], I[1], I[2]);
-  if (I[c] == 0 || I[c] == axis_len(cs, c)) { u.c[c][q] = 0.f; return; }
-  const long pc = cs.idx(I[0], I[1], I[2]);
-  const long step = c == 0 ? (long)cs.s1 * cs.s2 : (c == 1 ? cs.s2 : 1);
-  u.c[c][q] = (float)((double)u.c[c][q] - (x[pc] - x[pc - step]));
-}
-
 // End of fm_project_dc: an unconverged loop counts as a not-converged solve;
 // the state returns to plain solves (no floor, not done).
 __global__ void k_dc_finish(DevState* st) {
@@ -443,9 +450,10 @@ __global__ void k_dc_finish(DevState* st) {
   st->dc_tol = 0.0;
 }
 
-// subtract_grad_p + apply_bc (3D/mgpcg.py:401-427)
-template <typename T, int D>
-__global__ void k_subgrad_bc(fm_grid g, const T* __restrict__ p, MacW<T> u) {
+// subtract_grad_p + apply_bc (3D/mgpcg.py:401-427), 2D.  T: the pressure's type (FP64 for
+// a defect-corrected FP32 velocity).
+template <typename T, typename U>
+__global__ void k_subgrad_bc2(fm_grid g, const T* __restrict__ p, MacW<U> u) {
   pdl_begin();
   const int c = blockIdx.y;
   const Shape fs = face_shape(g, c);
@@ -456,8 +464,8 @@ __global__ void k_subgrad_bc(fm_grid g, const T* __restrict__ p, MacW<T> u) {
   unflatten(fs, q, I[0], I[1], I[2]);
   if (I[c] == 0 || I[c] == axis_len(cs, c)) { u.c[c][q] = 0; return; }
   const long pc = cs.idx(I[0], I[1], I[2]);
-  const long step = c == 0 ? (long)cs.s1 * cs.s2 : (c == 1 ? cs.s2 : 1);
-  u.c[c][q] -= p[pc] - p[pc - step];
+  const long step = c == 0 ? cs.s1 : 1;
+  u.c[c][q] = (U)((T)u.c[c][q] - (p[pc] - p[pc - step]));
 }
 
 // ---------------------------------------------------------------------------
@@ -836,6 +844,611 @@ __global__ void k_prolong(Shape sf, Shape sc, SF* __restrict__ zf, const SC* __r
   }
 }
 
+// ---------------------------------------------------------------------------
+// 3D: columns of planes
+// ---------------------------------------------------------------------------
+// The fine levels of a 3D solve live in the L2, and a kernel that reads the 7-point
+// neighbourhood of each cell by itself fetches every cell about four times and spends
+// most of its issue slots on indices.  The kernels below walk along axis 0 instead: a
+// thread owns a pair of cells (.., 2m), (.., 2m+1) and keeps the planes before and
+// after in registers, the neighbours along k come from the next lanes by shuffles,
+// those along j from the L1, and the loads of the next plane are issued before the
+// current one is used.  A block is 32 pairs x 8 rows, an item of work a stretch of
+// planes of such a tile, blocks take items in a stride (so that the reductions have at
+// most kRedBlocks partial sums).  Seven blocks fit an SM: the stretch is as long as
+// leaves about that many.  128^3 FP32, us, warm: last half-sweep with its inner product
+// 16.6 -> 9.2, A p and its inner product 12.9 -> 8.5, restriction 9.0 -> 7.5, prolongation
+// 9.0 -> 5.2, gradient subtraction 37.8 -> 14.4.  (A plain half-sweep gains nothing: 7.2 by
+// pairs of one plane, 9.3 walking with the walls worked out per plane.)
+struct Walk {
+  int tk, tj, planes, items;
+};
+constexpr int kWalkBX = 32, kWalkBY = 8, kWalkBlocks = 148 * 7;
+// over n0 planes, n1 rows, nk columns of the threads, in at most `most` items where
+// stretches of whole columns allow
+inline Walk walk_of(int n0, int n1, int nk, int most) {
+  Walk w;
+  w.tk = (nk + kWalkBX - 1) / kWalkBX;
+  w.tj = (n1 + kWalkBY - 1) / kWalkBY;
+  const long tiles = (long)w.tk * w.tj;
+  const int segs = tiles < most ? (int)(most / tiles) : 1;
+  w.planes = (n0 + segs - 1) / segs;
+  w.items = (int)(tiles * ((n0 + w.planes - 1) / w.planes));
+  return w;
+}
+inline Walk walk_pairs(const Shape& s, int most) { return walk_of(s.s0, s.s1, (s.s2 + 1) / 2, most); }
+constexpr dim3 kWalkBlock(kWalkBX, kWalkBY);
+__device__ __forceinline__ void walk_item(const Walk& w, int it, int n0, int& i0, int& i1, int& j, int& m) {
+  const int t = it / w.tk;
+  m = (it - t * w.tk) * kWalkBX + threadIdx.x;
+  const int seg = t / w.tj;
+  j = (t - seg * w.tj) * kWalkBY + threadIdx.y;
+  i0 = seg * w.planes;
+  i1 = min(i0 + w.planes, n0);
+}
+
+// How a pair of cells of a row is stored: one by one, by one aligned load (an even row
+// length and an aligned array), or by colour (below).
+enum { kOne = 0, kVec = 1, kSplit = 2 };
+// The pair at p; ha / hb: its cells exist (0 otherwise); oa: kSplit, the offset of
+// the first one's colour (0 or h), p then points at the pair in the first colour.
+template <int MODE, typename T, typename S>
+__device__ __forceinline__ void load_two(const S* p, bool ha, bool hb, T& a, T& b, int oa = 0, int h = 0) {
+  if constexpr (MODE == kVec) {
+    a = b = (T)0;
+    if (hb) {
+      if constexpr (std::is_same<S, __nv_bfloat16>::value) {
+        const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(p);
+        a = (T)__low2float(v), b = (T)__high2float(v);
+      } else {
+        using V = std::conditional_t<std::is_same<S, float>::value, float2, double2>;
+        const V v = *reinterpret_cast<const V*>(p);
+        a = (T)v.x, b = (T)v.y;
+      }
+    }
+  } else {
+    a = ha ? (T)to_c(p[MODE == kSplit ? oa : 0]) : (T)0;
+    b = hb ? (T)to_c(p[MODE == kSplit ? h - oa : 1]) : (T)0;
+  }
+}
+// neighbours of a cell within its plane
+__device__ __forceinline__ int plane_nd(const Shape& s, int j, int k) {
+  return 6 - (j == 0) - (j == s.s1 - 1) - (k == 0) - (k == s.s2 - 1);
+}
+inline bool two_aligned(const void* p, size_t elem, const Shape& s) {
+  return s.s2 % 2 == 0 && (uintptr_t)p % (2 * elem) == 0;
+}
+
+// smooth(l, phase) (3D/mgpcg.py:170-177), only the cells of colour `phase`, and
+// the partial sums of z.r over all cells.  The other colour's cell of a
+// pair is the +-i neighbour of the updated cells in the planes beside, and a +-k
+// neighbour of this plane's and of the next pair's updated cell; none of them is
+// written here, so loads may run ahead of the stores.  Which cell of the pair is
+// updated alternates with the planes and is the same for the whole warp (a row):
+// planes are taken by twos with it known at compile time, and what a column needs
+// of the walls is worked out once (with both done per plane the kernel is bound by
+// issue slots, 174 instructions a plane).
+template <typename T>
+__global__ void __launch_bounds__(kWalkBX* kWalkBY) k_smooth_dot_walk(Shape s, Walk w, const T* __restrict__ r, T* z,
+                                                                 int phase, double* __restrict__ part,
+                                                                 const DevState* st) {
+  pdl_begin();
+  if (st->done) return;
+  constexpr unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const long sj = s.s2, si = (long)s.s1 * s.s2;
+  double acc = 0;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int i0, i1, j, m;
+    walk_item(w, it, s.s0, i0, i1, j, m);
+    if (j >= s.s1) continue;  // the whole warp: a warp is one row
+    const int k0 = 2 * m;
+    // per cell of the pair: it exists, its +-j neighbours do, its k neighbour of another warp does
+    const bool kv[2] = {k0 < s.s2, k0 + 1 < s.s2};
+    const bool kp[2] = {kv[0] && j < s.s1 - 1, kv[1] && j < s.s1 - 1}, km[2] = {kv[0] && j > 0, kv[1] && j > 0};
+    const bool kf[2] = {kv[0] && lane == 0 && k0 > 0, lane == 31 && k0 + 2 < s.s2};
+    const int nd[2] = {plane_nd(s, j, k0), plane_nd(s, j, k0 + 1)};
+    const ClQuot<T> quot[2] = {ClQuot<T>(nd[0]), ClQuot<T>(nd[1])};
+    const long q = ((long)i0 * s.s1 + j) * s.s2 + k0;
+    T* zp = z + q;  // the pair in plane i
+    const T* rp = r + q;
+    struct Plane {
+      T o, jp, jm, r, ro, far;
+    };
+    // what the plane at zp needs, SH the updated cell: the other colour's cell (`in`:
+    // the plane exists), the +-j neighbours, the residual(s), the outer k neighbour
+    const auto fetch = [&](auto sh_, const T* zq, const T* rq, bool in, bool whole) {
+      constexpr int SH = decltype(sh_)::value;
+      Plane p;
+      p.o = in && kv[1 - SH] ? (zq[1 - SH]) : (T)0;
+      p.jp = whole && kp[SH] ? (zq[SH + sj]) : (T)0;
+      p.jm = whole && km[SH] ? (zq[SH - sj]) : (T)0;
+      p.r = whole && kv[SH] ? (rq[SH]) : (T)0;
+      p.ro = whole && kv[1 - SH] ? (rq[1 - SH]) : (T)0;
+      p.far = whole && kf[SH] ? (zq[SH ? 2 : -1]) : (T)0;
+      return p;
+    };
+    const auto walk = [&](auto first) {
+      constexpr int S0 = decltype(first)::value;
+      using A = std::integral_constant<int, S0>;
+      using B = std::integral_constant<int, 1 - S0>;
+      T om = i0 > 0 && kv[S0] ? (zp[S0 - si]) : (T)0;
+      Plane c = fetch(A(), zp, rp, true, true);
+      const auto step = [&](auto sh_, auto next_, int i) {
+        constexpr int SH = decltype(sh_)::value;
+        const Plane n = fetch(next_, zp + si, rp + si, i + 1 < s.s0, i + 1 < i1);
+        const T side = SH ? __shfl_down_sync(all, c.o, 1) : __shfl_up_sync(all, c.o, 1);
+        const T far = lane == (SH ? 31 : 0) ? c.far : side;
+        T nb = (T)0;
+        nb += n.o;
+        nb += om;
+        nb += c.jp;
+        nb += c.jm;
+        nb += SH ? far : c.o;
+        nb += SH ? c.o : far;
+        const T x = c.r + nb;
+        T v;
+        if (i > 0 && i < s.s0 - 1) {
+          v = quot[SH].fast(x);
+          if (quot[SH].template bad<true>(x)) v = quot[SH].slow(x);
+        } else {
+          v = div_nd(x, nd[SH] - (i == 0) - (i == s.s0 - 1));
+        }
+        if (kv[SH]) zp[SH] = v;
+        acc += kv[SH] ? (double)v * (double)c.r : 0.0;
+        acc += (double)c.o * (double)c.ro;
+        om = c.o;
+        c = n;
+        zp += si;
+        rp += si;
+      };
+      int i = i0;
+      for (; i + 1 < i1; i += 2) {
+        step(A(), B(), i);
+        step(B(), A(), i + 1);
+      }
+      if (i < i1) step(A(), B(), i);
+    };
+    if ((i0 + j + phase) & 1) walk(std::integral_constant<int, 1>());
+    else walk(std::integral_constant<int, 0>());
+  }
+  block_reduce2_2d(acc, 0.0, part + 2 * blockIdx.x);
+  walk_clear(part);
+}
+
+// Ap = A p and the partial sums of p.Ap
+template <typename T, int MODE>
+__global__ void __launch_bounds__(kWalkBX* kWalkBY) k_Ap_walk(Shape s, Walk w, const T* __restrict__ p,
+                                                             T* __restrict__ Ap, double* __restrict__ part,
+                                                             const DevState* st) {
+  pdl_begin();
+  if (st->done) return;
+  constexpr unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const long sj = s.s2, si = (long)s.s1 * s.s2;
+  double acc = 0;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int i0, i1, j, m;
+    walk_item(w, it, s.s0, i0, i1, j, m);
+    if (j >= s.s1) continue;  // the whole warp
+    const int k0 = 2 * m;
+    const bool ha = k0 < s.s2, hb = k0 + 1 < s.s2;
+    const bool pa = ha && j < s.s1 - 1, pb = hb && j < s.s1 - 1, la = ha && j > 0, lb = hb && j > 0;
+    const bool edge = (lane == 0 && ha && k0 > 0) || (lane == 31 && k0 + 2 < s.s2);
+    const int eo = lane == 0 ? -1 : 2;
+    const T nda = (T)plane_nd(s, j, k0), ndb = (T)plane_nd(s, j, k0 + 1);
+    const long q = ((long)i0 * s.s1 + j) * s.s2 + k0;
+    const T* pp = p + q;
+    T* ap = Ap + q;
+    struct Plane {
+      T a, b, pa, pb, ma, mb, far;  // the pair, its +j and -j pairs, the k neighbour outside the warp
+    };
+    const auto fetch = [&](const T* x, bool in, bool whole) {
+      Plane v;
+      load_two<MODE>(x, in && ha, in && hb, v.a, v.b);
+      load_two<MODE>(x + sj, whole && pa, whole && pb, v.pa, v.pb);
+      load_two<MODE>(x - sj, whole && la, whole && lb, v.ma, v.mb);
+      v.far = whole && edge ? x[eo] : (T)0;
+      return v;
+    };
+    T ma, mb;
+    load_two<MODE>(pp - si, i0 > 0 && ha, i0 > 0 && hb, ma, mb);
+    Plane c = fetch(pp, true, true);
+#pragma unroll 2
+    for (int i = i0; i < i1; ++i) {
+      const Plane n = fetch(pp + si, i + 1 < s.s0, i + 1 < i1);
+      const T up = __shfl_down_sync(all, c.a, 1), dn = __shfl_up_sync(all, c.b, 1);
+      const T left = lane == 0 ? c.far : dn, right = lane == 31 ? c.far : up;
+      T na = (T)0, nb = (T)0;
+      na += n.a, na += ma, na += c.pa, na += c.ma, na += c.b, na += left;
+      nb += n.b, nb += mb, nb += c.pb, nb += c.mb, nb += right, nb += c.a;
+      const T wall = (T)((i == 0) + (i == s.s0 - 1));
+      const T ra = rn_sub(rn_mul(nda - wall, c.a), na), rb = rn_sub(rn_mul(ndb - wall, c.b), nb);
+      if constexpr (MODE == kVec) {
+        using V = std::conditional_t<std::is_same<T, float>::value, float2, double2>;
+        if (hb) *reinterpret_cast<V*>(ap) = V{ra, rb};
+      } else {
+        if (ha) ap[0] = ra;
+        if (hb) ap[1] = rb;
+      }
+      acc += (double)c.a * (double)ra;  // a missing cell is 0
+      acc += (double)c.b * (double)rb;
+      ma = c.a, mb = c.b;
+      c = n;
+      pp += si;
+      ap += si;
+    }
+  }
+  block_reduce2_2d(acc, 0.0, part + 2 * blockIdx.x);
+  walk_clear(part);
+}
+
+// restrict(l) (3D/mgpcg.py:157-163): a thread owns the coarse cell of a pair column and
+// two rows, and walks the fine planes; children in the order of the gather.
+// out_split: the coarse level is stored by colour.
+template <typename T, typename SF, typename SC, int MODE>
+__global__ void __launch_bounds__(kWalkBX* kWalkBY) k_restrict_walk(Shape sf, Shape sc, Walk w,
+                                                                   const SF* __restrict__ rf,
+                                                                   const SF* __restrict__ zf, SC* __restrict__ rc,
+                                                                   int out_split, const DevState* st) {
+  pdl_begin();
+  if (st->done) return;
+  constexpr unsigned all = 0xffffffffu;
+  const T scale = (T)1.0 / (T)2.0;
+  const int lane = threadIdx.x;
+  const long sj = sf.s2, si = (long)sf.s1 * sf.s2;
+  const int h = sf.s2 / 2;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int I0, I1, J, K;
+    walk_item(w, it, sc.s0, I0, I1, J, K);
+    if (J >= sc.s1) continue;  // the whole warp
+    const bool on = K < sc.s2;  // then the fine pairs exist
+    const int k0 = 2 * K, j0 = 2 * J;
+    const bool jl = on && j0 > 0, jh = on && j0 + 2 < sf.s1;
+    const bool el = on && lane == 0 && k0 > 0;
+    const bool er = on && k0 + 2 < sf.s2 && (lane == 31 || K + 1 >= sc.s2);  // a last odd cell has no pair
+    T nd[2][2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) nd[d][0] = (T)plane_nd(sf, j0 + d, k0), nd[d][1] = (T)plane_nd(sf, j0 + d, k0 + 1);
+    // by colour: the first cell of a pair in row j0 + d of plane i has colour (d + i) & 1 (j0 and k0 are even)
+    const long q = ((long)(2 * I0) * sf.s1 + j0) * sf.s2 + (MODE == kSplit ? K : k0);
+    const SF* zp = zf + q;
+    const SF* rp = rf + q;
+    SC* out = rc + ((long)I0 * sc.s1 + J) * sc.s2;
+    T ma[2], mb[2], ca[2], cb[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      load_two<MODE>(zp - si + d * sj, on && I0 > 0, on && I0 > 0, ma[d], mb[d], d ? 0 : h, h);
+      load_two<MODE>(zp + d * sj, on, on, ca[d], cb[d], d ? h : 0, h);
+    }
+    for (int I = I0; I < I1; ++I) {
+      T acc = (T)0;
+#pragma unroll
+      for (int di = 0; di < 2; ++di) {
+        const int i = 2 * I + di;
+        T na[2], nb[2], xa[2], xb[2], ra[2], rb[2], eL[2], eR[2];
+        const bool up = on && i + 1 < sf.s0;
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const int oa = ((d + di) & 1) ? h : 0;  // the first cell's colour
+          load_two<MODE>(zp + si + d * sj, up, up, na[d], nb[d], h - oa, h);
+          load_two<MODE>(rp + d * sj, on, on, ra[d], rb[d], oa, h);
+          eL[d] = el ? (T)to_c(zp[d * sj + (MODE == kSplit ? h - oa - 1 : -1)]) : (T)0;
+          eR[d] = er ? (T)to_c(zp[d * sj + (MODE == kSplit ? oa + 1 : 2)]) : (T)0;
+        }
+        load_two<MODE>(zp - sj, jl, jl, xa[0], xb[0], di ? 0 : h, h);
+        load_two<MODE>(zp + 2 * sj, jh, jh, xa[1], xb[1], di ? h : 0, h);
+        const T wall = (T)((i == 0) + (i == sf.s0 - 1));
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {  // row j0 + d
+          T left = __shfl_up_sync(all, cb[d], 1), right = __shfl_down_sync(all, ca[d], 1);
+          if (lane == 0) left = eL[d];
+          if (lane == 31 || er) right = eR[d];
+          const T pa = d == 0 ? ca[1] : xa[1], pb = d == 0 ? cb[1] : xb[1];  // +j
+          const T la = d == 0 ? xa[0] : ca[0], lb = d == 0 ? xb[0] : cb[0];  // -j
+          T sa = (T)0, sb = (T)0;
+          sa += na[d], sa += ma[d], sa += pa, sa += la, sa += cb[d], sa += left;
+          sb += nb[d], sb += mb[d], sb += pb, sb += lb, sb += right, sb += ca[d];
+          const T ga = rn_sub(ra[d], rn_sub(rn_mul(nd[d][0] - wall, ca[d]), sa));
+          const T gb = rn_sub(rb[d], rn_sub(rn_mul(nd[d][1] - wall, cb[d]), sb));
+          acc = rn_add(acc, rn_mul(ga, scale));
+          acc = rn_add(acc, rn_mul(gb, scale));
+        }
+#pragma unroll
+        for (int d = 0; d < 2; ++d) ma[d] = ca[d], mb[d] = cb[d], ca[d] = na[d], cb[d] = nb[d];
+        zp += si;
+        rp += si;
+      }
+      if (on) out[out_split ? ((I + J + K) & 1) * (sc.s2 / 2) + (K >> 1) : K] = to_s<SC>(acc);
+      out += (long)sc.s1 * sc.s2;
+    }
+  }
+}
+
+// prolongate(l) (3D/mgpcg.py:165-168), a coarse cell's column of fine pairs per thread;
+// in_split: the coarse level is stored by colour
+template <typename T, typename SF, typename SC, int MODE>
+__global__ void __launch_bounds__(kWalkBX* kWalkBY) k_prolong_walk(Shape sf, Shape sc, Walk w, SF* __restrict__ zf,
+                                                                  const SC* __restrict__ zc, int in_split,
+                                                                  const DevState* st) {
+  pdl_begin();
+  if (st->done) return;
+  const unsigned si = (unsigned)sf.s1 * sf.s2;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int i0, i1, j, m;
+    walk_item(w, it, sf.s0, i0, i1, j, m);
+    const int k0 = 2 * m;
+    if (j >= sf.s1 || k0 >= sf.s2) continue;
+    const bool hb = k0 + 1 < sf.s2;
+    unsigned q = ((unsigned)i0 * sf.s1 + j) * sf.s2 + (MODE == kSplit ? m : k0);
+    const SC* const zcol = zc + (j >> 1) * (unsigned)sc.s2;
+    const int h = sf.s2 / 2;
+    const unsigned sci = (unsigned)sc.s1 * sc.s2;
+#pragma unroll 4
+    for (int i = i0; i < i1; ++i, q += si) {
+      const int I = i >> 1, at = in_split ? ((I + (j >> 1) + m) & 1) * (sc.s2 / 2) + (m >> 1) : m;
+      const T c = (T)to_c(zcol[I * sci + at]);
+      const int oa = MODE == kSplit && ((i + j) & 1) ? h : 0, ob = MODE == kSplit ? h - oa : 1;
+      T a, b;
+      load_two<MODE>(zf + q, true, hb, a, b, oa, h);
+      zf[q + oa] = to_s<SF>(a + c);
+      if (hb) zf[q + ob] = to_s<SF>(b + c);
+    }
+  }
+}
+
+// subtract_grad_p + apply_bc (3D/mgpcg.py:401-427): a column of cells per thread, each with
+// its three low faces (and the high ones at the walls)
+template <typename T, typename U>
+__global__ void __launch_bounds__(kWalkBX* kWalkBY) k_subgrad_walk(Shape s, Walk w, const T* __restrict__ p,
+                                                                  U* __restrict__ ux, U* __restrict__ uy,
+                                                                  U* __restrict__ uz) {
+  pdl_begin();
+  const unsigned si = (unsigned)s.s1 * s.s2;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int i0, i1, j, k;
+    walk_item(w, it, s.s0, i0, i1, j, k);
+    if (j >= s.s1 || k >= s.s2) continue;
+    unsigned q = ((unsigned)i0 * s.s1 + j) * s.s2 + k;
+    unsigned qy = ((unsigned)i0 * (s.s1 + 1) + j) * s.s2 + k;
+    unsigned qz = ((unsigned)i0 * s.s1 + j) * (s.s2 + 1) + k;
+    T below = i0 > 0 ? p[q - si] : (T)0;
+#pragma unroll 4
+    for (int i = i0; i < i1; ++i) {
+      const T c = p[q];
+      const U vy = j > 0 ? (U)((T)uy[qy] - (c - p[q - s.s2])) : (U)0;
+      const U vz = k > 0 ? (U)((T)uz[qz] - (c - p[q - 1])) : (U)0;
+      ux[q] = i > 0 ? (U)((T)ux[q] - (c - below)) : (U)0;
+      uy[qy] = vy;
+      uz[qz] = vz;
+      if (i == s.s0 - 1) ux[q + si] = (U)0;
+      if (j == s.s1 - 1) uy[qy + s.s2] = (U)0;
+      if (k == s.s2 - 1) uz[qz + 1] = (U)0;
+      below = c;
+      q += si;
+      qy += (unsigned)(s.s1 + 1) * s.s2;
+      qz += (unsigned)s.s1 * (s.s2 + 1);
+    }
+  }
+}
+template <typename T, typename U>
+static void launch_subgrad(const fm_grid& g, const T* p, const MacW<U>& u, cudaStream_t s) {
+  if (g.dim == 3) {
+    const Shape cs = cell_shape(g);
+    const Walk w = walk_of(cs.s0, cs.s1, cs.s2, kWalkBlocks);
+    launch_pdl(k_subgrad_walk<T, U>, (unsigned)w.items, kWalkBlock, 0, s, cs, w, p, u.c[0], u.c[1], u.c[2]);
+  } else {
+    const long f0 = face_shape(g, 0).size(), f1 = face_shape(g, 1).size(), n = f0 > f1 ? f0 : f1;
+    launch_pdl(k_subgrad_bc2<T, U>, dim3((unsigned)((n + 255) / 256), 2), 256, 0, s, g, p, u);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 3D, levels stored by colour
+// ---------------------------------------------------------------------------
+// Whatever the kernel, an interleaved half-sweep at 128^3 takes 7.2 us: it moves 25 MB
+// (z and r whole, z back) through the L2, of which it uses half.  Where every per-level
+// row has 16 n cells the V-cycle therefore stores z and r of those levels by colour
+// within the row: cell k of colour c = (i + j + k) & 1 at c s2 / 2 + (k >> 1).  The
+// first sweep splits the residual (into rs), the last one writes z in natural order (into
+// A p's array, which is free then), so that the rest of the solver does not see it; a
+// half-sweep moves 12.6 MB.  A thread updates 8 cells of a row: 16-byte loads of the
+// other colour in the row and its four neighbours and of the residual.  Within a
+// row the neighbours of the cell at m with sigma = (i + j + c) & 1 are the other colour's
+// m + sigma (k + 1) and m + sigma - 1.  Lanes of a warp have rows of the same parity,
+// so that sigma is the same for all.  128^3 FP32, us, warm: half-sweep 7.2 -> 5.2, first
+// 7.8 -> 8.6 (it writes the split residual too), last with its inner product 16.6 -> 8.8,
+// restriction 7.5 -> 9.2 and prolongation 5.2 -> 6.1 (walking); 64^3 in BF16 all as before (3.2 a
+// half-sweep: a launch).  A V-cycle with three smoothing steps: 220 -> 180.
+constexpr int kRow = 8;
+inline bool split_fits(const Shape& s) { return s.s2 % (2 * kRow) == 0; }
+struct Rows {
+  int lx, by, gx, gy, items;  // threads per row (log2), rows per block, blocks along the row and along j, blocks
+};
+inline Rows rows_of(const Shape& s, int threads) {
+  Rows w;
+  const int chunks = s.s2 / (2 * kRow);
+  w.lx = 0;
+  while (w.lx < 5 && (1 << w.lx) < chunks) ++w.lx;
+  w.by = threads >> w.lx;
+  w.gx = (chunks + (1 << w.lx) - 1) >> w.lx;
+  w.gy = (s.s1 + w.by - 1) / w.by;
+  w.items = w.gx * w.gy * s.s0;
+  return w;
+}
+// block b's row group: plane i, row j, first m of a colour; false past the end.  A
+// warp holds rows a multiple of the number of warps (even) apart.
+__device__ __forceinline__ bool rows_at(const Rows& w, const Shape& s, int b, int& i, int& j, int& m) {
+  const int tx = threadIdx.x & ((1 << w.lx) - 1), ty = threadIdx.x >> w.lx;
+  const int rpw = 32 >> w.lx, nw = blockDim.x >> 5;  // rows per warp, warps
+  const int bx = w.gx == 1 ? 0 : b % w.gx, t = w.gx == 1 ? b : b / w.gx;
+  i = t / w.gy;
+  j = (t - i * w.gy) * w.by + (ty >> (5 - w.lx)) + (ty & (rpw - 1)) * nw;
+  m = ((bx << w.lx) + tx) * kRow;
+  return j < s.s1 && 2 * m < s.s2;
+}
+// 8 cells, 16-byte aligned (zeros when `on` is false)
+template <typename T>
+__device__ __forceinline__ void load_row(const float* p, bool on, T* v) {
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+  if (on) a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+template <typename T>
+__device__ __forceinline__ void load_row(const double* p, bool on, T* v) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    double2 a = make_double2(0.0, 0.0);
+    if (on) a = reinterpret_cast<const double2*>(p)[m];
+    v[2 * m] = (T)a.x, v[2 * m + 1] = (T)a.y;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void load_row(const __nv_bfloat16* p, bool on, T* v) {
+  uint4 a = make_uint4(0, 0, 0, 0);
+  if (on) a = *reinterpret_cast<const uint4*>(p);
+  const unsigned x[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+  for (int m = 0; m < 4; ++m) v[2 * m] = (T)__uint_as_float(x[m] << 16), v[2 * m + 1] = (T)__uint_as_float(x[m] & 0xffff0000u);
+}
+template <typename T>
+__device__ __forceinline__ void store_row(float* p, const T* v) {
+  reinterpret_cast<float4*>(p)[0] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4((float)v[4], (float)v[5], (float)v[6], (float)v[7]);
+}
+template <typename T>
+__device__ __forceinline__ void store_row(double* p, const T* v) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) reinterpret_cast<double2*>(p)[m] = make_double2((double)v[2 * m], (double)v[2 * m + 1]);
+}
+template <typename T>
+__device__ __forceinline__ void store_row(__nv_bfloat16* p, const T* v) {
+  unsigned x[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const __nv_bfloat162 h = __halves2bfloat162(to_s<__nv_bfloat16>(v[2 * m]), to_s<__nv_bfloat16>(v[2 * m + 1]));
+    x[m] = *reinterpret_cast<const unsigned*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(x[0], x[1], x[2], x[3]);
+}
+
+// smooth(l, phase) (3D/mgpcg.py:170-177) of a level stored by colour.  OUT: instead of into
+// z the updated cells go, with the other colour's, to `out` in natural order, and
+// the partial sums of z.r over all cells to part (blocks take several items then).
+template <typename T, typename S, bool OUT>
+__global__ void __launch_bounds__(OUT ? 256 : 128) k_smooth_split(Shape s, Rows w, const S* __restrict__ r, S* z,
+                                                                int phase, S* __restrict__ out,
+                                                                double* __restrict__ part, const DevState* st) {
+  pdl_begin();
+  if (st->done) return;
+  const long sj = s.s2, si = (long)s.s1 * s.s2;
+  const int h = s.s2 / 2;
+  double acc = 0;
+  for (int it = blockIdx.x; it < w.items; it += gridDim.x) {
+    int i, j, m;
+    if (!rows_at(w, s, it, i, j, m)) continue;
+    const long row = (long)i * si + (long)j * sj;
+    const S* const o = z + row + (1 - phase) * h + m;  // the other colour
+    const int nd = 6 - (i == 0) - (i == s.s0 - 1) - (j == 0) - (j == s.s1 - 1);
+    T x[kRow], ip[kRow], im[kRow], jp[kRow], jm[kRow], rv[kRow], ro[kRow], v[kRow];
+    // the neighbour rows' other colour has the same place in the row
+    load_row(o, true, x);
+    load_row(o + si, i < s.s0 - 1, ip);
+    load_row(o - si, i > 0, im);
+    load_row(o + sj, j < s.s1 - 1, jp);
+    load_row(o - sj, j > 0, jm);
+    load_row(r + row + phase * h + m, true, rv);
+    if (OUT) load_row(r + row + (1 - phase) * h + m, true, ro);
+    const auto body = [&](auto sg_) {
+      constexpr int SG = decltype(sg_)::value, E = SG ? kRow - 1 : 0;  // E: the cell whose outer k neighbour is another thread's
+      const bool wall = SG ? m + kRow >= h : m == 0;
+      const T far = wall ? (T)0 : (T)to_c(o[SG ? kRow : -1]);
+      const ClQuot<T> quot(nd), quot_e(nd - wall);
+      T y[kRow];
+      bool bad = false;
+#pragma unroll
+      for (int a = 0; a < kRow; ++a) {
+        T nb = (T)0;
+        nb += ip[a];
+        nb += im[a];
+        nb += jp[a];
+        nb += jm[a];
+        nb += SG ? (a == kRow - 1 ? far : x[a == kRow - 1 ? a : a + 1]) : x[a];
+        nb += SG ? x[a] : (a == 0 ? far : x[a == 0 ? a : a - 1]);
+        y[a] = rv[a] + nb;
+        v[a] = a == E ? quot_e.fast(y[a]) : quot.fast(y[a]);
+        bad |= a == E ? quot_e.template bad<true>(y[a]) : quot.template bad<true>(y[a]);
+      }
+      if (bad) {
+#pragma unroll
+        for (int a = 0; a < kRow; ++a) v[a] = div_nd(y[a], a == E ? nd - wall : nd);
+      }
+      if constexpr (OUT) {
+        T nat[2 * kRow];  // cell 2 a + SG is the updated one
+#pragma unroll
+        for (int a = 0; a < kRow; ++a) {
+          nat[2 * a + SG] = v[a];
+          nat[2 * a + 1 - SG] = x[a];
+          acc += (double)v[a] * (double)rv[a];
+          acc += (double)x[a] * (double)ro[a];
+        }
+        store_row(out + row + 2 * m, nat);
+        store_row(out + row + 2 * m + kRow, nat + kRow);
+      } else {
+        store_row(z + row + phase * h + m, v);
+      }
+    };
+    if ((i + j + phase) & 1) body(std::integral_constant<int, 1>());
+    else body(std::integral_constant<int, 0>());
+  }
+  if constexpr (OUT) {
+    block_reduce2(acc, 0.0, part + 2 * blockIdx.x);
+    walk_clear(part);
+  }
+}
+
+// First red sweep from z == 0 (the black cells need no zeros: the next half-sweep
+// writes them from the red ones).  rn: the residual in natural order (the finest
+// level), stored by colour into r; recentre: less its mean, also in rn.
+template <typename T, typename S>
+__global__ void __launch_bounds__(128) k_first_split(Shape s, Rows w, S* __restrict__ rn, S* __restrict__ r,
+                                                     S* __restrict__ z, const DevState* st, int recenter) {
+  pdl_begin();
+  if (st->done) return;
+  int i, j, m;
+  if (!rows_at(w, s, blockIdx.x, i, j, m)) return;
+  const int h = s.s2 / 2;
+  const long row = ((long)i * s.s1 + j) * s.s2;
+  const int sg = (i + j) & 1;  // the red cell of a pair
+  T red[kRow];
+  if (rn) {
+    T nat[2 * kRow], black[kRow];
+    load_row(rn + row + 2 * m, true, nat);
+    load_row(rn + row + 2 * m + kRow, true, nat + kRow);
+    if (recenter) {
+      const T mean = (T)st->mean;
+#pragma unroll
+      for (int a = 0; a < 2 * kRow; ++a) nat[a] = nat[a] - mean;
+      store_row(rn + row + 2 * m, nat);
+      store_row(rn + row + 2 * m + kRow, nat + kRow);
+    }
+#pragma unroll
+    for (int a = 0; a < kRow; ++a) {
+      red[a] = sg ? nat[2 * a + 1] : nat[2 * a];
+      black[a] = sg ? nat[2 * a] : nat[2 * a + 1];
+    }
+    store_row(r + row + m, red);
+    store_row(r + row + h + m, black);
+  } else {
+    load_row(r + row + m, true, red);
+  }
+  const int nd = 6 - (i == 0) - (i == s.s0 - 1) - (j == 0) - (j == s.s1 - 1);
+#pragma unroll
+  for (int a = 0; a < kRow; ++a)
+    red[a] = div_nd(red[a], nd - (a == 0 && m == 0 && !sg) - (a == kRow - 1 && m + kRow >= h && sg));
+  store_row(z + row + m, red);
+}
+
 // Bottom smoothing on the coarsest level by one CTA in shared memory.
 // z starts at zero (the reference zero-fills before restricting).
 template <typename T, int D>
@@ -943,6 +1556,7 @@ struct fm_mgpcg {
   void* x;
   void* p;
   void* Ap;
+  void* rs;        // the finest residual by colour, for V-cycles on levels stored so (null: natural order)
   double* part;
   DevState* st;
   DevState* h_st;  // pinned
@@ -1030,7 +1644,10 @@ static void launch_coarse(fm_mgpcg* S, cudaStream_t s) {
             (T*)S->z[S->lc], (const DevState*)S->st);
 }
 
-// One V-cycle (apply_preconditioner, 3D/mgpcg.py:187-205) on r[0] -> z[0].
+// Where a V-cycle leaves its result, in natural order.
+static void* zout(const fm_mgpcg* S) { return S->rs ? S->Ap : S->z[0]; }
+
+// One V-cycle (apply_preconditioner, 3D/mgpcg.py:187-205) on r[0] -> zout.
 // recenter: subtract st->mean from r[0] first (fused into the first sweep);
 // dot_last: the last fine sweep also writes z.r block partials.
 template <typename T, int D>
@@ -1051,16 +1668,26 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
   // level storage: T, or BF16 for levels 1 .. bf16_hi-1 (FP32 solvers with coarse_bf16)
   using BF = __nv_bfloat16;
   auto bf = [&](int l) { return std::is_same<T, float>::value && l >= 1 && l < S->bf16_hi; };
+  const bool split = D == 3 && S->rs;  // the per-level levels are stored by colour
+  auto rl = [&](int l) { return l == 0 && split ? (T*)S->rs : r[l]; };
   auto sweep = [&](int l, int phase) {
     const Shape sh = S->lv[l];
-    if (bf(l)) launch_pdl(k_smooth_pair<T, D, BF>, pair_grid(sh), pblk, 0, s, sh, (const BF*)S->r[l], (BF*)S->z[l], phase, S->st);
+    if (split) {
+      const Rows w = rows_of(sh, 128);
+      if (bf(l)) launch_pdl(k_smooth_split<T, BF, false>, (unsigned)w.items, 128, 0, s, sh, w, (const BF*)S->r[l], (BF*)S->z[l], phase, (BF*)nullptr, nullptr, S->st);
+      else launch_pdl(k_smooth_split<T, T, false>, (unsigned)w.items, 128, 0, s, sh, w, (const T*)rl(l), z[l], phase, (T*)nullptr, nullptr, S->st);
+    } else if (bf(l)) launch_pdl(k_smooth_pair<T, D, BF>, pair_grid(sh), pblk, 0, s, sh, (const BF*)S->r[l], (BF*)S->z[l], phase, S->st);
     else launch_pdl(k_smooth_pair<T, D>, pair_grid(sh), pblk, 0, s, sh, (const T*)r[l], z[l], phase, S->st);
   };
   for (int l = 0; l < lc; ++l) {
     const Shape sh = S->lv[l];
     const dim3 pg = pair_grid(sh);
     for (int it = 0; it < P.pre_post; ++it) {
-      if (it == 0) {
+      if (it == 0 && split) {
+        const Rows w = rows_of(sh, 128);
+        if (bf(l)) launch_pdl(k_first_split<T, BF>, (unsigned)w.items, 128, 0, s, sh, w, (BF*)nullptr, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
+        else launch_pdl(k_first_split<T, T>, (unsigned)w.items, 128, 0, s, sh, w, l == 0 ? r[0] : (T*)nullptr, rl(l), z[l], S->st, l == 0 && recenter ? 1 : 0);
+      } else if (it == 0) {
         if (bf(l)) launch_pdl(k_smooth_first_pair<T, D, BF>, pg, pblk, 0, s, sh, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
         else launch_pdl(k_smooth_first_pair<T, D>, pg, pblk, 0, s, sh, r[l], z[l], S->st, l == 0 && recenter ? 1 : 0);
       } else {
@@ -1069,15 +1696,31 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
       sweep(l, 1);
     }
     const Shape sc = S->lv[l + 1];
-    const unsigned rb = blocks_for(sc.size(), 256, cap);
-    if (bf(l) && bf(l + 1))
-      launch_pdl(k_restrict<T, D, BF, BF>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], (BF*)S->r[l + 1], S->st);
-    else if (bf(l))
-      launch_pdl(k_restrict<T, D, BF, T>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], r[l + 1], S->st);
-    else if (bf(l + 1))
-      launch_pdl(k_restrict<T, D, T, BF>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], (BF*)S->r[l + 1], S->st);
-    else
-      launch_pdl(k_restrict<T, D>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], r[l + 1], S->st);
+    if constexpr (D == 3) {
+      const Walk w = walk_of(sc.s0, sc.s1, sc.s2, kWalkBlocks);
+      auto go = [&](auto* rf, auto* zf, auto* rc) {
+        using SF = std::remove_pointer_t<decltype(rf)>;
+        const bool vec = two_aligned(rf, sizeof(SF), sh) && two_aligned(zf, sizeof(SF), sh);
+        const int out_split = split && l + 1 < lc;
+        using SC = std::remove_pointer_t<decltype(rc)>;
+        launch_pdl(split ? k_restrict_walk<T, SF, SC, kSplit> : (vec ? k_restrict_walk<T, SF, SC, kVec> : k_restrict_walk<T, SF, SC, kOne>),
+                   (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, (const SF*)rf, (const SF*)zf, rc, out_split, (const DevState*)S->st);
+      };
+      if (bf(l) && bf(l + 1)) go((BF*)S->r[l], (BF*)S->z[l], (BF*)S->r[l + 1]);
+      else if (bf(l)) go((BF*)S->r[l], (BF*)S->z[l], r[l + 1]);
+      else if (bf(l + 1)) go(rl(l), z[l], (BF*)S->r[l + 1]);
+      else go(rl(l), z[l], r[l + 1]);
+    } else {
+      const unsigned rb = blocks_for(sc.size(), 256, cap);
+      if (bf(l) && bf(l + 1))
+        launch_pdl(k_restrict<T, D, BF, BF>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], (BF*)S->r[l + 1], S->st);
+      else if (bf(l))
+        launch_pdl(k_restrict<T, D, BF, T>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], r[l + 1], S->st);
+      else if (bf(l + 1))
+        launch_pdl(k_restrict<T, D, T, BF>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], (BF*)S->r[l + 1], S->st);
+      else
+        launch_pdl(k_restrict<T, D>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], r[l + 1], S->st);
+    }
   }
   const Shape sb = S->lv[L - 1];
   if (S->lc > 0) {
@@ -1108,20 +1751,47 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
   for (int l = lc - 1; l >= 0; --l) {
     const Shape sh = S->lv[l];
     const Shape sc = S->lv[l + 1];
-    const unsigned nb = blocks_for(sh.size(), 256, cap);
-    if (bf(l) && bf(l + 1))
-      launch_pdl(k_prolong<T, D, BF, BF>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const BF*)S->z[l + 1], S->st);
-    else if (bf(l))
-      launch_pdl(k_prolong<T, D, BF, T>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const T*)z[l + 1], S->st);
-    else if (bf(l + 1))
-      launch_pdl(k_prolong<T, D, T, BF>, nb, 256, 0, s, sh, sc, z[l], (const BF*)S->z[l + 1], S->st);
-    else
-      launch_pdl(k_prolong<T, D>, nb, 256, 0, s, sh, sc, z[l], (const T*)z[l + 1], S->st);
+    if constexpr (D == 3) {
+      const Walk w = walk_pairs(sh, kWalkBlocks);
+      auto go = [&](auto* zf, auto* zc) {
+        using SF = std::remove_pointer_t<decltype(zf)>;
+        using SC = std::remove_pointer_t<decltype(zc)>;
+        const bool vec = two_aligned(zf, sizeof(SF), sh);
+        launch_pdl(split ? k_prolong_walk<T, SF, SC, kSplit> : (vec ? k_prolong_walk<T, SF, SC, kVec> : k_prolong_walk<T, SF, SC, kOne>),
+                   (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, zf, (const SC*)zc, (int)(split && l + 1 < lc),
+                   (const DevState*)S->st);
+      };
+      if (bf(l) && bf(l + 1)) go((BF*)S->z[l], (BF*)S->z[l + 1]);
+      else if (bf(l)) go((BF*)S->z[l], z[l + 1]);
+      else if (bf(l + 1)) go(z[l], (BF*)S->z[l + 1]);
+      else go(z[l], z[l + 1]);
+    } else {
+      const unsigned nb = blocks_for(sh.size(), 256, cap);
+      if (bf(l) && bf(l + 1))
+        launch_pdl(k_prolong<T, D, BF, BF>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const BF*)S->z[l + 1], S->st);
+      else if (bf(l))
+        launch_pdl(k_prolong<T, D, BF, T>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const T*)z[l + 1], S->st);
+      else if (bf(l + 1))
+        launch_pdl(k_prolong<T, D, T, BF>, nb, 256, 0, s, sh, sc, z[l], (const BF*)S->z[l + 1], S->st);
+      else
+        launch_pdl(k_prolong<T, D>, nb, 256, 0, s, sh, sc, z[l], (const T*)z[l + 1], S->st);
+    }
     for (int it = 0; it < P.pre_post; ++it) {
       sweep(l, 1);
-      const bool last = dot_last && l == 0 && it == P.pre_post - 1;
-      if (last) launch_pdl(k_smooth<T, D, true>, kRedBlocks, kRedThreads, 0, s, sh, r[l], z[l], 0, S->part, S->st);
-      else sweep(l, 0);
+      const bool end = l == 0 && it == P.pre_post - 1, last = dot_last && end;
+      if (end && split) {
+        const Rows w = rows_of(sh, 256);
+        launch_pdl(k_smooth_split<T, T, true>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), 256, 0, s, sh, w,
+                   (const T*)S->rs, z[0], 0, (T*)S->Ap, S->part, S->st);
+      } else if (!last) {
+        sweep(l, 0);
+      } else if constexpr (D == 3) {
+        const Walk w = walk_pairs(sh, kRedBlocks);
+        launch_pdl(k_smooth_dot_walk<T>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock, 0, s, sh, w,
+                   (const T*)r[l], z[l], 0, S->part, S->st);
+      } else {
+        launch_pdl(k_smooth<T, D, true>, kRedBlocks, kRedThreads, 0, s, sh, r[l], z[l], 0, S->part, S->st);
+      }
     }
   }
   if (dot_last && L == 1) {
@@ -1136,7 +1806,14 @@ template <typename T, int D>
 static void launch_step(fm_mgpcg* S, cudaStream_t s) {
   const Shape s0 = S->lv[0];
   const long n = s0.size();
-  launch_pdl(k_Ap_dot<T, D>, kRedBlocks, kRedThreads, 0, s, s0, (T*)S->p, (T*)S->Ap, S->part, S->st);
+  if constexpr (D == 3) {
+    const Walk w = walk_pairs(s0, kRedBlocks);
+    const bool vec = two_aligned(S->p, sizeof(T), s0) && two_aligned(S->Ap, sizeof(T), s0);
+    launch_pdl(vec ? k_Ap_walk<T, kVec> : k_Ap_walk<T, kOne>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock,
+               0, s, s0, w, (const T*)S->p, (T*)S->Ap, S->part, S->st);
+  } else {
+    launch_pdl(k_Ap_dot<T, D>, kRedBlocks, kRedThreads, 0, s, s0, (T*)S->p, (T*)S->Ap, S->part, S->st);
+  }
   launch_pdl(k_fin_alpha, 1, 256, 0, s, S->st, S->part, S->P.eps);
   launch_pdl(k_update_xr<T>, kRedBlocks, kRedThreads, 0, s, n, (T*)S->x, (T*)S->r[0], (T*)S->p, (T*)S->Ap,
              S->part, S->st);
@@ -1153,7 +1830,7 @@ static void launch_iteration(fm_mgpcg* S, cudaStream_t s) {
   const long n = S->lv[0].size();
   launch_vcycle<T, D>(S, s, true);
   launch_pdl(k_fin_beta, 1, 256, 0, s, S->st, S->part, S->P.eps, S->P.abs_tol, S->P.rel_tol, S->P.max_iters, 0);
-  launch_pdl(k_update_p<T>, blocks_for(n, 256, 148L * 16), 256, 0, s, n, (T*)S->p, (T*)S->z[0], S->st, 0);
+  launch_pdl(k_update_p<T>, blocks_for(n, 256, 148L * 16), 256, 0, s, n, (T*)S->p, (const T*)zout(S), S->st, 0);
   launch_step<T, D>(S, s);
 }
 
@@ -1165,7 +1842,7 @@ static void launch_prologue(fm_mgpcg* S, cudaStream_t s) {
   launch_pdl(k_fin_mean, 1, 256, 0, s, S->st, S->part, (double)n);
   launch_vcycle<T, D>(S, s, true);
   launch_pdl(k_fin_beta, 1, 256, 0, s, S->st, S->part, S->P.eps, S->P.abs_tol, S->P.rel_tol, S->P.max_iters, 1);
-  launch_pdl(k_update_p<T>, blocks_for(n, 256, 148L * 16), 256, 0, s, n, (T*)S->p, (T*)S->z[0], S->st, 1);
+  launch_pdl(k_update_p<T>, blocks_for(n, 256, 148L * 16), 256, 0, s, n, (T*)S->p, (const T*)zout(S), S->st, 1);
   launch_step<T, D>(S, s);
 }
 
@@ -1415,7 +2092,17 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
     ok = ok && cudaMalloc(&S->z[l], e * S->lv[l].size()) == cudaSuccess;
   }
   const long n0 = S->lv[0].size();
-  ok = ok && cudaMalloc(&S->x, es * n0) == cudaSuccess;
+  // 3D levels of 16 n cells a row are stored by colour: a second residual, in x's allocation; without the memory
+  // for it the levels stay in natural order
+  const int fine = S->lc > 0 ? S->lc : S->L - 1;
+  bool split = g->dim == 3 && !S->pcg_nc && P.pre_post > 0 && fine > 0;
+  for (int l = 0; l < fine; ++l) split = split && split_fits(S->lv[l]);
+  if (split && ok) {
+    const size_t xb = (es * n0 + 255) / 256 * 256;
+    if (cudaMalloc(&S->x, xb + es * n0) == cudaSuccess) S->rs = (char*)S->x + xb;
+    else cudaGetLastError(), S->x = nullptr;
+  }
+  if (!S->x) ok = ok && cudaMalloc(&S->x, es * n0) == cudaSuccess;
   if (!S->pcg_nc) {  // a cluster solve keeps p and A p in shared memory
     ok = ok && cudaMalloc(&S->p, es * n0) == cudaSuccess;
     ok = ok && cudaMalloc(&S->Ap, es * n0) == cudaSuccess;
@@ -1488,25 +2175,20 @@ int fm_project(fm_mgpcg* S, void* ux, void* uy, void* uz, void* p_out, void* str
   const fm_grid g = S->g;
   const long n = S->lv[0].size();
   int status;
-  long maxf = 0;
-  for (int c = 0; c < g.dim; ++c) maxf = face_shape(g, c).size() > maxf ? face_shape(g, c).size() : maxf;
-  dim3 fgrid((unsigned)((maxf + 255) / 256), (unsigned)g.dim, 1);
   if (S->dtype == FM_F32) {
     MacW<float> u{{(float*)ux, (float*)uy, (float*)uz}};
     if (g.dim == 3) launch_pdl(k_div_bc<float, 3>, kRedBlocks, kRedThreads, 0, s, g, u, (float*)S->r[0], (float*)S->x, S->part);
     else launch_pdl(k_div_bc<float, 2>, kRedBlocks, kRedThreads, 0, s, g, u, (float*)S->r[0], (float*)S->x, S->part);
     status = run_solve<float>(S, s, iters, rtr);
     if (status == FM_ERR_CUDA) return status;
-    if (g.dim == 3) launch_pdl(k_subgrad_bc<float, 3>, fgrid, 256, 0, s, g, (const float*)S->x, u);
-    else launch_pdl(k_subgrad_bc<float, 2>, fgrid, 256, 0, s, g, (const float*)S->x, u);
+    launch_subgrad(g, (const float*)S->x, u, s);
   } else {
     MacW<double> u{{(double*)ux, (double*)uy, (double*)uz}};
     if (g.dim == 3) launch_pdl(k_div_bc<double, 3>, kRedBlocks, kRedThreads, 0, s, g, u, (double*)S->r[0], (double*)S->x, S->part);
     else launch_pdl(k_div_bc<double, 2>, kRedBlocks, kRedThreads, 0, s, g, u, (double*)S->r[0], (double*)S->x, S->part);
     status = run_solve<double>(S, s, iters, rtr);
     if (status == FM_ERR_CUDA) return status;
-    if (g.dim == 3) launch_pdl(k_subgrad_bc<double, 3>, fgrid, 256, 0, s, g, (const double*)S->x, u);
-    else launch_pdl(k_subgrad_bc<double, 2>, fgrid, 256, 0, s, g, (const double*)S->x, u);
+    launch_subgrad(g, (const double*)S->x, u, s);
   }
   if (p_out) cudaMemcpyAsync(p_out, S->x, (S->dtype == FM_F32 ? 4 : 8) * n, cudaMemcpyDeviceToDevice, s);
   if (check_cuda()) return FM_ERR_CUDA;
@@ -1545,7 +2227,7 @@ int fm_mg_vcycle(fm_mgpcg* S, const void* r, void* z, void* stream) {
     if (S->g.dim == 3) launch_vcycle<double, 3>(S, s, false, false);
     else launch_vcycle<double, 2>(S, s, false, false);
   }
-  if (cudaMemcpyAsync(z, S->z[0], bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return FM_ERR_CUDA;
+  if (cudaMemcpyAsync(z, zout(S), bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return FM_ERR_CUDA;
   return check_cuda();
 }
 
@@ -1638,11 +2320,7 @@ int fm_project_dc(fm_mgpcg* S, void* ux, void* uy, void* uz, double* work, doubl
     launch_pdl(k_dc_update_g, nb, 256, 0, s, n, x, (const float*)S->x, (const DevState*)S->st);
     residual(2);
   }
-  long maxf = 0;
-  for (int c = 0; c < D; ++c) maxf = face_shape(g, c).size() > maxf ? face_shape(g, c).size() : maxf;
-  dim3 fgrid((unsigned)((maxf + 255) / 256), (unsigned)D, 1);
-  if (D == 3) launch_pdl(k_dc_subgrad<3>, fgrid, 256, 0, s, g, (const double*)x, u);
-  else launch_pdl(k_dc_subgrad<2>, fgrid, 256, 0, s, g, (const double*)x, u);
+  launch_subgrad(g, (const double*)x, u, s);
   launch_pdl(k_dc_finish, 1, 1, 0, s, S->st);
   if (p_out) cudaMemcpyAsync(p_out, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
   if (check_cuda()) return FM_ERR_CUDA;
@@ -1858,9 +2536,6 @@ extern "C" int fm_project_noalloc(const fm_grid* g, int dtype, const fm_mg_param
   cudaStream_t s = (cudaStream_t)stream;
   // the scratch keeps the previous call's contents: the solver state must start at zero
   if (cudaMemsetAsync(S.st, 0, sizeof(DevState), s) != cudaSuccess) return FM_ERR_CUDA;
-  long maxf = 0;
-  for (int c = 0; c < g->dim; ++c) maxf = face_shape(*g, c).size() > maxf ? face_shape(*g, c).size() : maxf;
-  dim3 fgrid((unsigned)((maxf + 255) / 256), (unsigned)g->dim, 1);
   const fm_grid gg = *g;
   int status;
   if (dtype == FM_F32) {
@@ -1869,16 +2544,14 @@ extern "C" int fm_project_noalloc(const fm_grid* g, int dtype, const fm_mg_param
     else launch_pdl(k_div_bc<float, 2>, kRedBlocks, kRedThreads, 0, s, gg, u, (float*)S.r[0], (float*)S.x, S.part);
     status = run_solve_direct<float>(&S, s, iters, rtr);
     if (status == FM_ERR_CUDA) return status;
-    if (gg.dim == 3) launch_pdl(k_subgrad_bc<float, 3>, fgrid, 256, 0, s, gg, (const float*)S.x, u);
-    else launch_pdl(k_subgrad_bc<float, 2>, fgrid, 256, 0, s, gg, (const float*)S.x, u);
+    launch_subgrad(gg, (const float*)S.x, u, s);
   } else {
     MacW<double> u{{(double*)ux, (double*)uy, (double*)uz}};
     if (gg.dim == 3) launch_pdl(k_div_bc<double, 3>, kRedBlocks, kRedThreads, 0, s, gg, u, (double*)S.r[0], (double*)S.x, S.part);
     else launch_pdl(k_div_bc<double, 2>, kRedBlocks, kRedThreads, 0, s, gg, u, (double*)S.r[0], (double*)S.x, S.part);
     status = run_solve_direct<double>(&S, s, iters, rtr);
     if (status == FM_ERR_CUDA) return status;
-    if (gg.dim == 3) launch_pdl(k_subgrad_bc<double, 3>, fgrid, 256, 0, s, gg, (const double*)S.x, u);
-    else launch_pdl(k_subgrad_bc<double, 2>, fgrid, 256, 0, s, gg, (const double*)S.x, u);
+    launch_subgrad(gg, (const double*)S.x, u, s);
   }
   if (check_cuda()) return FM_ERR_CUDA;
   return status;
