@@ -84,7 +84,8 @@ inline void launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
 
 // As launch(), with the programmatic-serialization attribute: the kernel's CTAs
 // may be scheduled before its stream predecessor finishes and wait for it in
-// pdl_begin().  Only for kernels whose first statement is pdl_begin().
+// pdl_begin().  Only for kernels that before pdl_begin() read nothing a kernel
+// launched after their handle's set-up writes, and write nothing but shared memory.
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   if (!g_pdl.load(std::memory_order_relaxed)) {

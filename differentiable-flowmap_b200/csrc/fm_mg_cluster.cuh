@@ -697,15 +697,15 @@ struct ClCta {
 template <typename T, int D, typename St>
 __global__ void __launch_bounds__(kClThreads, 1) k_mg_coarse(const ClArgs* __restrict__ args, const T* __restrict__ r_top,
                                                              T* __restrict__ z_top, const St* st) {
-  pdl_begin();
-  if (st->done) return;  // same value in every CTA of the cluster
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const ClArgs& a = cl_load_args(args);
   ClCta<T, D, false> C(a, (int)cl.block_rank(), (int)cl.num_blocks());
   const int l = a.l0, tid = threadIdx.x;
   const ClLevel& L = a.lv[l];
-  C.setup();
+  C.setup();  // of this CTA's own shared memory only: runs beside the kernel before (128^3 projection: 446 -> 443 us)
+  pdl_begin();
+  if (st->done) return;  // same value in every CTA of the cluster
   __syncthreads();
   // natural rows -> colour arrays (cell k of a row at m = k >> 1)
   const int rowlen = L.nin, nrows = C.planes(l) * L.rows;
@@ -795,8 +795,6 @@ template <typename T, int D, bool SOLID, typename Ctx>
 __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(const ClArgs* __restrict__ args, PcgParams P,
                                                                const T* __restrict__ r_in, T* __restrict__ x_out,
                                                                Ctx st) {
-  pdl_begin();
-  if (pcg_skip(st)) return;  // same value in every CTA of the cluster
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClSums sums;
@@ -815,8 +813,14 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(const ClArgs* __r
   const long g0 = (long)C.first_plane(0) * L.rows * L.nin;  // cell (2m) of pair e is at g0 + 2 e (even rows)
   const double ncell = (double)L.s.size();
   int turn = 0;
+  // the set-up writes this CTA's own shared memory and reads constants of the handle: it
+  // runs beside the kernel before, unless there are masks, which a kernel packs (256^2
+  // projection: 316 -> 313 us)
+  if (SOLID) pdl_begin();
   C.setup();
   for (int q = tid; q < 2 * zsz; q += kClThreads) p[q] = 0;
+  if (!SOLID) pdl_begin();
+  if (pcg_skip(st)) return;  // same value in every CTA of the cluster
   cl_cluster_sync();  // heads and zeroed ghosts everywhere before the first push
   const uint32_t p_lo = rank > 0 ? cl_remote(p, rank - 1) : 0, p_hi = rank < nc - 1 ? cl_remote(p, rank + 1) : 0;
   const ClRun& R0 = cl_head()->run[0];
@@ -1026,15 +1030,25 @@ inline cudaError_t cl_launch(void (*k)(KArgs...), int nc, size_t smem, cudaStrea
   return e;
 }
 
-// The device copy of a geometry (once per handle).
-inline ClArgs* cl_upload(const ClArgs& a) {
-  ClArgs* d = nullptr;
-  if (cudaMalloc((void**)&d, sizeof(ClArgs)) != cudaSuccess) return nullptr;
-  if (cudaMemcpy(d, &a, sizeof(ClArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(d);
-    return nullptr;
-  }
-  return d;
+// Whether the device runs `kernel` as a cluster of nc CTAs with this much shared memory.
+template <typename Kernel>
+inline bool cl_enable(Kernel kernel, int nc, size_t smem) {
+  if (!raise_smem_limit(kernel, smem)) return false;
+  if (nc > 8 && cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nc, 1, 1);
+  cfg.blockDim = dim3(kClThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)nc;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  return cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
 }
 
 // Plans a whole solve in one cluster: returns the CTAs, or 0 where it does not
@@ -1053,21 +1067,7 @@ inline int cl_plan_pcg(ClArgs& a, Kernel kernel, const Shape* lv, int L, const f
     if (smem > kClMaxSmem && nc < kClMaxNC) continue;
     if (smem > kClMaxSmem) smem = cl_layout(a, lv, 0, ld, L, dim, es, nc, true, solid, false);
     if (smem > kClMaxSmem) return 0;
-    if (!raise_smem_limit(kernel, smem)) break;
-    if (nc > 8 && cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) break;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)nc, 1, 1);
-    cfg.blockDim = dim3(kClThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)nc;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) break;
+    if (!cl_enable(kernel, nc, smem)) break;
     a.pre_post = P.pre_post;
     a.bottom = P.bottom;
     a.bottom_mode = P.bottom_mode;

@@ -1583,7 +1583,7 @@ struct fm_mgpcg {
 namespace fm {
 
 // Picks the finest level lc >= 1 from which the rest of the V-cycle runs as one
-// cluster launch: level lc split into nc <= 8 slabs of an even number of planes,
+// cluster launch: level lc split into nc <= 8 slabs (enable_coarse_kernel: 16) of an even number of planes,
 // every slab and every deeper level at most 4096 cells (two pairs per thread:
 // beyond that a per-level launch spread over the chip is faster).  lc = -1 when
 // no level qualifies (the V-cycle launches per level).
@@ -1619,9 +1619,25 @@ static void plan_coarse(fm_mgpcg* S, size_t es) {
   }
 }
 
+// Makes the plan launchable.  Slabs of more than one pair a thread are halved over 16 CTAs
+// (beyond the portable cluster size) where the device takes such a cluster: 32^3 on
+// 16 CTAs instead of 8, FP32, a 128^3 projection: 443 -> 434 us.
 template <typename T, int D>
-static bool enable_coarse_kernel(size_t smem) {
-  return raise_smem_limit(k_mg_coarse<T, D, DevState>, smem);
+static bool enable_coarse_kernel(fm_mgpcg* S, size_t es) {
+  const Shape t = S->lv[S->lc];
+  const int nc = 2 * kCoarseMaxNC;
+  if (S->nc == kCoarseMaxNC && t.s0 % (2 * nc) == 0 && coarse_pairs(t, D, t.s0 / S->nc) > kClThreads) {
+    ClArgs a = S->coarse;
+    const size_t smem = cl_layout(a, S->lv, S->lc, S->lc + 1, S->L, D, es, nc, false, false);
+    if (smem > 0 && smem <= kClMaxSmem && cl_enable(k_mg_coarse<T, D, DevState>, nc, smem)) {
+      S->coarse = a;
+      S->nc = nc;
+      S->coarse_smem = smem;
+      return true;
+    }
+    cudaGetLastError();
+  }
+  return raise_smem_limit(k_mg_coarse<T, D, DevState>, S->coarse_smem);
 }
 
 template <typename T, int D>
@@ -2070,10 +2086,8 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
   // coarse levels in one cluster launch where they fit
   plan_coarse(S, es);
   if (S->lc > 0) {
-    const bool en = dtype == FM_F32 ? (g->dim == 3 ? enable_coarse_kernel<float, 3>(S->coarse_smem)
-                                                   : enable_coarse_kernel<float, 2>(S->coarse_smem))
-                                    : (g->dim == 3 ? enable_coarse_kernel<double, 3>(S->coarse_smem)
-                                                   : enable_coarse_kernel<double, 2>(S->coarse_smem));
+    const bool en = dtype == FM_F32 ? (g->dim == 3 ? enable_coarse_kernel<float, 3>(S, es) : enable_coarse_kernel<float, 2>(S, es))
+                                    : (g->dim == 3 ? enable_coarse_kernel<double, 3>(S, es) : enable_coarse_kernel<double, 2>(S, es));
     if (!en) {
       cudaGetLastError();
       S->lc = -1;

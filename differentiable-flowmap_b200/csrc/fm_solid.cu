@@ -993,15 +993,20 @@ template <typename T, int D>
 static bool plan_cluster(fm_solid* S) {
   S->pcg_nc = cl_plan_pcg(S->pcg, k_pcg_cluster<T, D, true, Ctx>, S->sh, S->levels, S->P, D, sizeof(T), true,
                           &S->pcg_smem);
-  bool ok = true;
-  for (int l = 0; S->pcg_nc && l < S->levels; ++l) {
+  if (!S->pcg_nc) return true;
+  // the geometry and the levels' masks in one allocation
+  constexpr size_t kHead = (sizeof(ClArgs) + 255) / 256 * 256;
+  size_t off[kClMaxLevels], bytes = kHead;
+  for (int l = 0; l < S->levels; ++l) {
     const Shape& sh = S->sh[l];
-    const long pairs = (long)sh.s0 * (D == 3 ? sh.s1 : 1) * (((D == 3 ? sh.s2 : sh.s1) + 1) / 2);
-    ok = ok && cudaMalloc((void**)&S->msk[l], sizeof(uint16_t) * pairs) == cudaSuccess;
-    S->pcg.msk[l] = S->msk[l];
+    off[l] = bytes;
+    bytes += (sizeof(uint16_t) * sh.s0 * (D == 3 ? sh.s1 : 1) * (((D == 3 ? sh.s2 : sh.s1) + 1) / 2) + 255) / 256 * 256;
   }
-  if (ok && S->pcg_nc) ok = (S->d_pcg = cl_upload(S->pcg)) != nullptr;
-  return ok;
+  char* base = nullptr;
+  if (cudaMalloc((void**)&base, bytes) != cudaSuccess) return false;
+  S->d_pcg = (ClArgs*)base;
+  for (int l = 0; l < S->levels; ++l) S->pcg.msk[l] = S->msk[l] = (uint16_t*)(base + off[l]);
+  return cudaMemcpy(S->d_pcg, &S->pcg, sizeof(ClArgs), cudaMemcpyHostToDevice) == cudaSuccess;
 }
 
 }  // namespace solid
@@ -1015,7 +1020,6 @@ int fm_solid_destroy(fm_solid* S) {
     cudaFree(S->r[l]);
     cudaFree(S->z[l]);
     cudaFree(S->fl[l]);
-    cudaFree(S->msk[l]);
   }
   cudaFree(S->x);
   cudaFree(S->p);
