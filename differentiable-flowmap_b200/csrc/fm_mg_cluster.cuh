@@ -178,6 +178,8 @@ __device__ __forceinline__ T cl_nb(int zo, int o, int s, int si, int sj, unsigne
   return nb;
 }
 
+__device__ __forceinline__ void cl_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cl_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cl_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -719,6 +721,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_mg_coarse(const ClArgs* __res
   }
   cl_cluster_sync();  // heads and zeroed ghosts everywhere before the first push
   C.vcycle();
+  // No CTA exits while another may still send to it: where every wait succeeds none
+  // can, but a CTA whose wait gave up runs ahead of its neighbours.  The stores
+  // below overlap the barrier.
+  cl_cluster_arrive();
   const T* z = C.z(l);
   for (int q = tid; q < nrows * rowlen; q += kClThreads) {
     const int row = L.dnin(q), k = q - row * rowlen;
@@ -727,6 +733,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_mg_coarse(const ClArgs* __res
     const T v = z[c * L.zsz() + (p + 1) * L.si + (D == 3 ? (j + 1) * L.sj : 0) + (k >> 1) + 1];
     z_top[g0 + q] = cl_head()->failed ? (T)nan("") : v;  // a wait that gave up ends the solve as non-finite
   }
+  cl_cluster_wait();
 }
 
 // ---------------------------------------------------------------------------
