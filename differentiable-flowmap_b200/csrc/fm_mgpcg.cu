@@ -2140,6 +2140,8 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
   ok = ok && cudaMallocHost(&S->h_st, sizeof(DevState)) == cudaSuccess;
   ok = ok && cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) == cudaSuccess;
   if (ok) ok = cudaMemset(S->st, 0, sizeof(DevState)) == cudaSuccess;
+  // both may still be under way; the first solve may come on a stream that the default one does not order
+  if (ok) ok = cudaStreamSynchronize(nullptr) == cudaSuccess;
   const long nb = S->lv[S->L - 1].size();
   const size_t smem = 2 * es * nb;
   if (ok && smem <= 200 * 1024 && nb <= kBottomMaxCells) {

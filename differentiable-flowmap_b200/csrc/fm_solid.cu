@@ -1117,6 +1117,7 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
   } else {
     for (int l = 0; l < P.levels; ++l) cudaMemset(S->fl[l], 1, S->sh[l].size());
     solid::pack_masks(S, nullptr);
+    cudaStreamSynchronize(nullptr);  // the first solve may come on a stream that the default one does not order
   }
   *out = S;
   return check_cuda();
