@@ -38,8 +38,8 @@
 //    other axes combined once per (column, Gaussian), four faces per shared load.
 //    The cull is a superset of the exact test.  3000 Gaussians of radius 1..9 cells
 //    on 128^3 in FP32: 289 us with the cull in FP64 and scalar table loads, 210 us now.
-//  * k_gauss_grad: one CTA per Gaussian over its support; short stretches of
-//    faces are summed in registers of the run's type and flushed to FP64;
+//  * k_gauss_grad: one CTA per Gaussian over its support; what a lane sums of one
+//    short stretch of faces is of the run's type, everything beyond it FP64;
 //    fixed-order warp-shuffle + shared-memory reduction, so the result is
 //    deterministic (the reference's atomics are not).  Gaussians with r <= 0 or a
 //    support longer than the table along the columns take a per-face path in the
@@ -55,7 +55,6 @@ constexpr int kGfThreads = 256;
 constexpr int kGfWarps = kGfThreads / 32;
 constexpr int kGfMaxN = 1 << 24;
 constexpr int kGfTab = 256;   // table capacity of the adjoint kernel (faces of an axis)
-constexpr int kGfFlush = 32;  // faces per lane after which its sums go to FP64
 
 // Tiles of the force kernel; the column axis is D-1.  SEG: faces per thread
 // along it (one segment per thread: 3D 9*8 + 8*9 + 8*8 = 208, 2D 17*4 + 16*5 = 148).
@@ -361,7 +360,7 @@ template <typename T> struct alignas(16) GfTask {
   unsigned rowst;   // a step along the middle axis
   short q0, last;   // last: of the 8 faces within the range
   short ma, mb, mlast, cc;
-  T d0, sq0, ex0;
+  T d0, sq0;
 };
 
 // The Gaussian that block b takes: a one-to-one map that puts wide supports
@@ -429,11 +428,15 @@ __device__ __forceinline__ int gf_order(int b, int n, const T* __restrict__ ir) 
 // is 8 faces of the column axis (k in 3D, j in 2D; contiguous in memory) at one
 // index of the outer axis; its warp walks, 4 faces at a time, the stretch of the
 // middle axis that the ball reaches there.  Every thread prepares one task, then
-// the warps take them in turn.  The column's factors stay in registers, the
-// middle axis' come from shared memory.  Sums of the run's type are flushed to
-// FP64 once they hold kGfFlush faces.  3000 Gaussians of radius 1..9 cells on 128^3
-// in FP32: 334 us with a lane per column (strided loads, 32 unequal columns per
-// warp) and 206 us now.
+// the warps take them in turn.  The factor of the outer and the column axis stays
+// in a register, the middle axis' come from shared memory.  A lane's sums over its
+// share of one task are of the run's type, their products with the offsets and the
+// sums over tasks are FP64, and a weight is the product of two factors: three (a
+// table entry per axis, whose roundings all faces of a plane share) put the FP32 sums
+// 1.2 to 1.4 times further from 64 bits.
+// 3000 Gaussians of radius 1..9 cells on 128^3 in FP32: 334 us with a lane per column
+// (strided loads, 32 unequal columns per warp), 206 us with three factors and FP32 sums
+// of up to 32 faces and more, 211 us now.
 template <typename T, int D>
 __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
     k_gauss_grad(fm_grid g, T dx, int n, const T* __restrict__ cen, const T* __restrict__ ir, const T* __restrict__ str,
@@ -490,23 +493,23 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
   const auto extent = [&](int cc, int a) { return s_len[a][cc == a]; };
   const auto cols = [&](int cc) { return r > (T)0 && extent(cc, CA) <= kGfTab; };
   const int mlen = max(s_len[MA][0], s_len[MA][1]);
-  T S = (T)0, S0 = (T)0, Sm = (T)0, Sc = (T)0, E = (T)0, E0 = (T)0, Em = (T)0, Ec = (T)0;
-  int held = 0, hc = 0;  // faces per lane in these sums, and their component
+  // one component's sums, and which one's
+  double S = 0.0, S0 = 0.0, Sm = 0.0, Sc = 0.0, E = 0.0, E0 = 0.0, Em = 0.0, Ec = 0.0;
+  int hc = -1;
   const auto flush = [&]() {
     T sc = s[0];
 #pragma unroll
     for (int cc = 0; cc < D; ++cc)
       if (hc == cc) {
         sc = s[cc];
-        v[cc] += (double)S;
-        v[2 * D + cc] += 2.0 * (double)sc * (double)E;
+        v[cc] += S;
+        v[2 * D + cc] += 2.0 * (double)sc * E;
       }
     const double k1 = 2.0 * (double)sc * (double)r, k2 = 2.0 * (double)sc * k1;
-    if (D == 3) v[D] += k1 * (double)S0, v[3 * D] += k2 * (double)E0;
-    v[D + MA] += k1 * (double)Sm, v[3 * D + MA] += k2 * (double)Em;
-    v[D + CA] += k1 * (double)Sc, v[3 * D + CA] += k2 * (double)Ec;
-    S = S0 = Sm = Sc = E = E0 = Em = Ec = (T)0;
-    held = 0;
+    if (D == 3) v[D] += k1 * S0, v[3 * D] += k2 * E0;
+    v[D + MA] += k1 * Sm, v[3 * D + MA] += k2 * Em;
+    v[D + CA] += k1 * Sc, v[3 * D + CA] += k2 * Ec;
+    S = S0 = Sm = Sc = E = E0 = Em = Ec = 0.0;
   };
   for (int m0 = 0; m0 < mlen && r > (T)0; m0 += kGfTab) {  // the middle axis in slabs of the table's length
     if (m0 > 0) __syncthreads();
@@ -535,14 +538,13 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
         const int tt = t - (cc == 0 ? 0 : (cc == 1 ? first[1] : first[2 < D ? 2 : 1]));
         const int ecol = extent(cc, CA), ms = min(kGfTab, extent(cc, MA) - m0);
         const int chunks = (ecol + LC - 1) / LC, o = tt / chunks, q0 = (tt - o * chunks) * LC;
-        GfAxis<T> out = {(T)0, (T)0, (T)1, (T)0};
-        if (D == 3) out = gf_axis<T>(start(cc, 0) + o, cc == 0, dx, c[0], r);
+        const T d0 = D == 3 ? rn_sub(gf_pos<T>(start(cc, 0) + o, cc == 0, dx), c[0]) : (T)0, sq0 = rn_mul(d0, d0);
         // the stretch that the ball reaches at the chunk's nearest face, widened
         // to whole indices; the centre in the slab's indices
         const T za = rn_sub(gf_pos<T>(start(cc, CA) + q0, cc == CA, dx), c[CA]);
         const T zb = rn_sub(gf_pos<T>(start(cc, CA) + min(q0 + LC, ecol) - 1, cc == CA, dx), c[CA]);
         const T zm = za > (T)0 ? za : (zb < (T)0 ? zb : (T)0);
-        const T rest = thi - out.sq - zm * zm;
+        const T rest = thi - sq0 - zm * zm;
         const T half = sqrt(rest) * inv + (T)0.01;
         const T cm = -rn_sub(gf_pos<T>(start(cc, MA) + m0, cc == MA, dx), c[MA]) * inv;
         const T mlo = D == 3 ? (T)0 : (T)(o * kStretch);
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
         k.rowst = D == 3 ? fs.s2 : fs.s1;
         k.q0 = (short)q0, k.last = (short)(min(q0 + LC, ecol) - 1 - q0), k.cc = (short)cc;
         k.ma = (short)ma, k.mb = (short)mb, k.mlast = (short)(ms - 1);
-        k.d0 = out.dp, k.sq0 = out.sq, k.ex0 = out.ex;
+        k.d0 = d0, k.sq0 = sq0;
         s_task[threadIdx.x] = k;
       }
       __syncthreads();
@@ -569,18 +571,19 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
         const GfTask<T> k = s_task[t];
         if (k.ma > k.mb) continue;
         const int cc = k.cc;
-        if (held >= kGfFlush || (cc != hc && held > 0)) flush();
-        hc = cc;
-        held += (k.mb - k.ma) / LM + UN;
+        if (cc != hc) {
+          if (hc >= 0) flush();
+          hc = cc;
+        }
         const int lc = min(lane & (LC - 1), (int)k.last);
         const GfAxis<T> col = t_col[cc == CA][k.q0 + lc];
         const T zsq = lc == (lane & (LC - 1)) ? col.sq : (T)INFINITY;  // past the end: outside
-        const T eoc = k.ex0 * col.ex;
+        const T eoc = D == 3 ? exp(-rn_mul(rn_add(k.sq0, col.sq), r)) : col.ex;
         const T* row = k.row + lc;
         const int mlast = k.mlast;
         const unsigned rowst = k.rowst;
         const GfAxis<T>* const mid = t_mid[cc == MA];
-        T P = (T)0, Q = (T)0;
+        T P = (T)0, Pm = (T)0, Q = (T)0, Qm = (T)0;
         for (int m = k.ma + lane / LC; m - lane / LC <= k.mb; m += PAD) {
           T av[UN], s2[UN], e[UN], dm[UN];
           bool in[UN], near = false;
@@ -608,19 +611,20 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
           for (int h = 0; h < UN; ++h) {  // selects: a NaN outside stays out
             const T ea = in[h] ? e[h] * av[h] : (T)0, e2 = in[h] ? e[h] * e[h] : (T)0;
             P += ea;
-            Sm += ea * dm[h];
+            Pm += ea * dm[h];
             Q += e2;
-            Em += e2 * dm[h];
+            Qm += e2 * dm[h];
           }
         }
-        S += P, Sc += col.dp * P;
-        E += Q, Ec += col.dp * Q;
-        if (D == 3) S0 += k.d0 * P, E0 += k.d0 * Q;
+        const double p = P, q = Q, dc = col.dp;
+        S += p, Sm += (double)Pm, Sc += dc * p;
+        E += q, Em += (double)Qm, Ec += dc * q;
+        if (D == 3) S0 += (double)k.d0 * p, E0 += (double)k.d0 * q;
       }
       __syncthreads();  // the tasks' last readers are done
     }
   }
-  if (held > 0) flush();
+  if (hc >= 0) flush();
   if (!none) {
 #pragma unroll
     for (int cc = 0; cc < D; ++cc) {
