@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(kGfThreads) k_gauss_force(fm_grid g, T dx, int
   }
 }
 
-// Face-index range along one axis within [lo, hi] (in cells; the bounds are
-// widened by a hundredth of a cell, far above their rounding).
+// Face-index range along one axis within [lo, hi] (in cells, widened by more than
+// the rounding of a face's position).
 __device__ __forceinline__ void gf_axis_range(double lo, double hi, bool face_axis, int len, int& i0, int& i1) {
   const double off = face_axis ? 0.0 : 0.5;
   const double a = fmax(ceil(lo - off), 0.0), b = fmin(floor(hi - off), (double)(len - 1));
@@ -471,7 +471,11 @@ __global__ void __launch_bounds__(kGfThreads, sizeof(T) == 4 ? 4 : 2)
     const int a = threadIdx.x >> 1, v = threadIdx.x & 1;
     double lo = -1.0, hi = 1e9;
     if (r > (T)0) {
-      const double R = sqrt(5.0 / (double)r) * (1.0 + kGfMargin) + 0.01 * (double)dx;
+      // a face's position and its offset from the centre are rounded in the run's type: by up to
+      // 2^-23 of the axis in FP32, 0.02 cells at 150000
+      const double ulp = sizeof(T) == 4 ? 0x1p-22 : 0x1p-51;
+      const double slack = 0.01 + ulp * (a == 0 ? g.n[0] : (a == 1 ? g.n[1] : g.n[2]));
+      const double R = sqrt(5.0 / (double)r) * (1.0 + kGfMargin) + slack * (double)dx;
       const double x = (double)(a == 0 ? c[0] : (a == 1 ? c[1] : c[CA]));
       lo = (x - R) / (double)dx;
       hi = (x + R) / (double)dx;
