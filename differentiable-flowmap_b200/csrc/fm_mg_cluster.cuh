@@ -530,6 +530,13 @@ struct ClCta {
   template <bool DIST>
   __device__ __forceinline__ void smooth(int l, int first, int halves, bool zero, int nthr) {
     if (halves == 0) return;
+    if (!SOLID && a.lv[l].s.size() == 1) {  // no neighbours: r / 0, as everywhere (the quotients below leave it out)
+      if (tid == 0) {
+        const int o = a.lv[l].si + (D == 3 ? a.lv[l].sj : 0) + 1;
+        z(l)[o] = div_nd(r(l)[o - a.lv[l].si], 0);
+      }
+      return;  // the caller ends the level with a barrier
+    }
     const int n = npairs(l);
     if (n <= nthr) phase = cl_smooth_u<T, D, SOLID, DIST, 1>(l, first, halves, zero, nthr, phase);
     else if (sizeof(T) == 4 && n <= 2 * nthr) phase = cl_smooth_u<T, D, SOLID, DIST, 2>(l, first, halves, zero, nthr, phase);
