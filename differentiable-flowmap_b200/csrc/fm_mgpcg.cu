@@ -1543,6 +1543,8 @@ __device__ __forceinline__ void pcg_finish(DevState* st, const PcgOutcome& R) {
 
 }  // namespace fm
 
+#include "fm_mg_ring.cuh"
+
 using namespace fm;
 
 struct fm_mgpcg {
@@ -1571,7 +1573,8 @@ struct fm_mgpcg {
   int lc;                      // levels lc .. L-1 run as one cluster launch (<= 0: per-level launches)
   int nc;                      // CTAs in that cluster
   size_t coarse_smem;
-  ClArgs coarse;               // its geometry
+  ClArgs coarse;               // its geometry: k_mg_coarse (3D FP32) ...
+  RingArgs ring;               // ... or k_mg_ring
   ClArgs* d_coarse;
   int pcg_nc;                  // CTAs of the cluster that runs a whole solve (0: the solve is a sequence of launches)
   size_t pcg_smem;
@@ -1583,32 +1586,64 @@ struct fm_mgpcg {
 namespace fm {
 
 // Picks the finest level lc >= 1 from which the rest of the V-cycle runs as one
-// cluster launch: level lc split into nc <= 8 slabs (enable_coarse_kernel: 16) of an even number of planes,
-// every slab and every deeper level at most 4096 cells (two pairs per thread:
+// cluster launch: level lc split into nc <= 8 slabs (enable_coarse: 16) of an even number of
+// planes, every slab and every deeper level at most 4096 cells (two pairs per thread:
 // beyond that a per-level launch spread over the chip is faster).  lc = -1 when
 // no level qualifies (the V-cycle launches per level).
 constexpr int kCoarseMaxNC = 8;
 constexpr long kCoarseMaxPairs = 2 * kClThreads;
+static_assert(kRingThreads == kClThreads && kRingPPT == 2, "one rule for both kernels");
+
+// Which kernel that is (fm_mg_ring.cuh has the figures).
+template <typename T, int D>
+constexpr bool kPushCoarse = D == 3 && sizeof(T) == 4;
 
 static long coarse_pairs(const Shape& s, int dim, int planes) {
   const long nin = dim == 3 ? s.s2 : s.s1;
   return (long)planes * (dim == 3 ? s.s1 : 1) * ((nin + 1) / 2);
 }
+static long coarse_ring(const Shape& s, int dim, int planes) {
+  return (long)planes * (s.s1 + 2) * (dim == 3 ? s.s2 + 2 : 1);
+}
 
-static void plan_coarse(fm_mgpcg* S, size_t es) {
+// k_mg_ring's shared memory for level lc on nc CTAs: slab, then CTA 0's deep levels (compact r, zero-ringed z).
+static size_t ring_layout(RingArgs& a, const fm_mgpcg* S, int lc, int nc, size_t es) {
+  const int dim = S->g.dim;
+  long off = 0;
+  for (int l = 0; l < S->L; ++l) {
+    const Shape& t = S->lv[l];
+    a.lv[l] = t;
+    a.roff[l] = a.zoff[l] = 0;
+    if (l <= lc) continue;
+    a.roff[l] = (int)off;
+    a.zoff[l] = (int)(off + t.size());
+    off += t.size() + coarse_ring(t, dim, t.s0 + 2);
+  }
+  a.lc = lc;
+  a.L = S->L;
+  a.pre_post = S->P.pre_post;
+  a.bottom = S->P.bottom;
+  a.bottom_mode = S->P.bottom_mode;
+  const Shape& t = S->lv[lc];
+  const int planes = t.s0 / nc;
+  return es * (size_t)(off + coarse_ring(t, dim, planes + 2) + (long)planes * t.s1 * t.s2);
+}
+
+template <typename T, int D>
+static void plan_coarse(fm_mgpcg* S) {
   S->lc = -1;
   S->nc = 0;
   S->coarse_smem = 0;
-  const int dim = S->g.dim;
   for (int l = 1; l < S->L - 1; ++l) {
     const Shape t = S->lv[l];
     int nc = kCoarseMaxNC;
     while (nc > 1 && t.s0 % (2 * nc) != 0) nc >>= 1;
-    if (t.s0 % (2 * nc) != 0 || coarse_pairs(t, dim, t.s0 / nc) > kCoarseMaxPairs) continue;
+    if (t.s0 % (2 * nc) != 0 || coarse_pairs(t, D, t.s0 / nc) > kCoarseMaxPairs) continue;
     bool fits = true;
-    for (int m = l + 1; m < S->L; ++m) fits = fits && coarse_pairs(S->lv[m], dim, S->lv[m].s0) <= kCoarseMaxPairs;
-    const size_t smem = cl_layout(S->coarse, S->lv, l, l + 1, S->L, dim, es, nc, false, false);
-    if (!fits || smem == 0 || smem > kClMaxSmem) continue;
+    for (int m = l + 1; m < S->L; ++m) fits = fits && coarse_pairs(S->lv[m], D, S->lv[m].s0) <= kCoarseMaxPairs;
+    const size_t smem = kPushCoarse<T, D> ? cl_layout(S->coarse, S->lv, l, l + 1, S->L, D, sizeof(T), nc, false, false)
+                                          : ring_layout(S->ring, S, l, nc, sizeof(T));
+    if (!fits || smem == 0 || smem > (kPushCoarse<T, D> ? kClMaxSmem : 200 * 1024)) continue;
     S->lc = l;
     S->nc = nc;
     S->coarse_smem = smem;
@@ -1623,21 +1658,35 @@ static void plan_coarse(fm_mgpcg* S, size_t es) {
 // (beyond the portable cluster size) where the device takes such a cluster: 32^3 on
 // 16 CTAs instead of 8, FP32, a 128^3 projection: 443 -> 434 us.
 template <typename T, int D>
-static bool enable_coarse_kernel(fm_mgpcg* S, size_t es) {
-  const Shape t = S->lv[S->lc];
-  const int nc = 2 * kCoarseMaxNC;
-  if (S->nc == kCoarseMaxNC && t.s0 % (2 * nc) == 0 && coarse_pairs(t, D, t.s0 / S->nc) > kClThreads) {
-    ClArgs a = S->coarse;
-    const size_t smem = cl_layout(a, S->lv, S->lc, S->lc + 1, S->L, D, es, nc, false, false);
-    if (smem > 0 && smem <= kClMaxSmem && cl_enable(k_mg_coarse<T, D, DevState>, nc, smem)) {
-      S->coarse = a;
-      S->nc = nc;
-      S->coarse_smem = smem;
-      return true;
+static bool enable_coarse(fm_mgpcg* S) {
+  if constexpr (kPushCoarse<T, D>) {
+    const Shape t = S->lv[S->lc];
+    const int nc = 2 * kCoarseMaxNC;
+    if (S->nc == kCoarseMaxNC && t.s0 % (2 * nc) == 0 && coarse_pairs(t, D, t.s0 / S->nc) > kClThreads) {
+      ClArgs a = S->coarse;
+      const size_t smem = cl_layout(a, S->lv, S->lc, S->lc + 1, S->L, D, sizeof(T), nc, false, false);
+      if (smem > 0 && smem <= kClMaxSmem && cl_enable(k_mg_coarse<T, D, DevState>, nc, smem)) {
+        S->coarse = a;
+        S->nc = nc;
+        S->coarse_smem = smem;
+        return true;
+      }
+      cudaGetLastError();
     }
-    cudaGetLastError();
+    return raise_smem_limit(k_mg_coarse<T, D, DevState>, S->coarse_smem);
+  } else {
+    return raise_smem_limit(k_mg_ring<T, D>, S->coarse_smem);
   }
-  return raise_smem_limit(k_mg_coarse<T, D, DevState>, S->coarse_smem);
+}
+
+// The coarse levels in one cluster launch where they fit.
+template <typename T, int D>
+static void plan_coarse_t(fm_mgpcg* S) {
+  plan_coarse<T, D>(S);
+  if (S->lc > 0 && !enable_coarse<T, D>(S)) {
+    cudaGetLastError();
+    S->lc = -1;
+  }
 }
 
 template <typename T, int D>
@@ -1653,11 +1702,18 @@ static inline unsigned blocks_for(long n, int threads, long cap) {
   return (unsigned)b;
 }
 
-// Levels lc .. L-1 of the V-cycle as one cluster launch (fm_mg_cluster.cuh).
+// Levels lc .. L-1 of the V-cycle as one cluster launch.
 template <typename T, int D>
 static void launch_coarse(fm_mgpcg* S, cudaStream_t s) {
-  cl_launch(k_mg_coarse<T, D, DevState>, S->nc, S->coarse_smem, s, (const ClArgs*)S->d_coarse, (const T*)S->r[S->lc],
-            (T*)S->z[S->lc], (const DevState*)S->st);
+  if constexpr (kPushCoarse<T, D>) {
+    cl_launch(k_mg_coarse<T, D, DevState>, S->nc, S->coarse_smem, s, (const ClArgs*)S->d_coarse, (const T*)S->r[S->lc],
+              (T*)S->z[S->lc], (const DevState*)S->st);
+  } else {
+    RingArgs a = S->ring;
+    a.r_top = S->r[S->lc];
+    a.z_top = S->z[S->lc];
+    cl_launch(k_mg_ring<T, D>, S->nc, S->coarse_smem, s, a, (const DevState*)S->st);
+  }
 }
 
 // Where a V-cycle leaves its result, in natural order.
@@ -2083,16 +2139,8 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
     sh.s2 = g->dim == 3 ? (g->n[2] >> l) : 1;
     S->lv[l] = sh;
   }
-  // coarse levels in one cluster launch where they fit
-  plan_coarse(S, es);
-  if (S->lc > 0) {
-    const bool en = dtype == FM_F32 ? (g->dim == 3 ? enable_coarse_kernel<float, 3>(S, es) : enable_coarse_kernel<float, 2>(S, es))
-                                    : (g->dim == 3 ? enable_coarse_kernel<double, 3>(S, es) : enable_coarse_kernel<double, 2>(S, es));
-    if (!en) {
-      cudaGetLastError();
-      S->lc = -1;
-    }
-  }
+  if (dtype == FM_F32) g->dim == 3 ? plan_coarse_t<float, 3>(S) : plan_coarse_t<float, 2>(S);
+  else g->dim == 3 ? plan_coarse_t<double, 3>(S) : plan_coarse_t<double, 2>(S);
   // BF16 storage for the per-level coarse levels 1 .. lc-1 (needs the cluster path)
   S->bf16_hi = (P.coarse_bf16 && S->lc > 1) ? S->lc : 0;
   // a grid that fits one cluster is solved in one launch (with BF16 levels it keeps those)
