@@ -1248,11 +1248,11 @@ static void launch_subgrad(const fm_grid& g, const T* p, const MacW<U>& u, cudaS
 // ---------------------------------------------------------------------------
 // Whatever the kernel, an interleaved half-sweep at 128^3 takes 7.2 us: it moves 25 MB
 // (z and r whole, z back) through the L2, of which it uses half.  Where every per-level
-// row has 16 n cells the V-cycle therefore stores z and r of those levels by colour
-// within the row: cell k of colour c = (i + j + k) & 1 at c s2 / 2 + (k >> 1).  The
-// first sweep splits the residual (into rs), the last one writes z in natural order (into
-// A p's array, which is free then), so that the rest of the solver does not see it; a
-// half-sweep moves 12.6 MB.  A thread updates 8 cells of a row: 16-byte loads of the
+// row has 16 n cells the V-cycle of a large FP32 solver therefore stores z and r of those
+// levels by colour within the row: cell k of colour c = (i + j + k) & 1 at c s2 / 2 +
+// (k >> 1).  The first sweep splits the residual (into rs), the last one writes z in natural
+// order (into A p's array, which is free then), so that the rest of the solver does not see
+// it; a half-sweep moves 12.6 MB.  A thread updates 8 cells of a row: 16-byte loads of the
 // other colour in the row and its four neighbours and of the residual.  Within a
 // row the neighbours of the cell at m with sigma = (i + j + c) & 1 are the other colour's
 // m + sigma (k + 1) and m + sigma - 1.  Lanes of a warp have rows of the same parity,
@@ -1261,6 +1261,11 @@ static void launch_subgrad(const fm_grid& g, const T* p, const MacW<U>& u, cudaS
 // restriction 7.5 -> 9.2 and prolongation 5.2 -> 6.1 (walking); 64^3 in BF16 all as before (3.2 a
 // half-sweep: a launch).  A V-cycle with three smoothing steps: 220 -> 180.
 constexpr int kRow = 8;
+// FP32 solvers of at least this many cells.  Projections of five iterations by colour and in
+// natural order, us: 48^3 439 and 418, 64^3 508 and 499, 64x96x128 625 and 611, 96^3 699 and
+// 702, 128^3 897 and 926 (on less, eight cells a thread leave too few threads); FP64 64^3
+// 682 and 604, 128^3 1555 and 1253 (a half-sweep is then bound by its divisions).
+constexpr long kSplitCells = 850000;
 inline bool split_fits(const Shape& s) { return s.s2 % (2 * kRow) == 0; }
 struct Rows {
   int lx, by, gx, gy, items;  // threads per row (log2), rows per block, blocks along the row and along j, blocks
@@ -1295,15 +1300,6 @@ __device__ __forceinline__ void load_row(const float* p, bool on, T* v) {
   v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
 template <typename T>
-__device__ __forceinline__ void load_row(const double* p, bool on, T* v) {
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    double2 a = make_double2(0.0, 0.0);
-    if (on) a = reinterpret_cast<const double2*>(p)[m];
-    v[2 * m] = (T)a.x, v[2 * m + 1] = (T)a.y;
-  }
-}
-template <typename T>
 __device__ __forceinline__ void load_row(const __nv_bfloat16* p, bool on, T* v) {
   uint4 a = make_uint4(0, 0, 0, 0);
   if (on) a = *reinterpret_cast<const uint4*>(p);
@@ -1315,11 +1311,6 @@ template <typename T>
 __device__ __forceinline__ void store_row(float* p, const T* v) {
   reinterpret_cast<float4*>(p)[0] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
   reinterpret_cast<float4*>(p)[1] = make_float4((float)v[4], (float)v[5], (float)v[6], (float)v[7]);
-}
-template <typename T>
-__device__ __forceinline__ void store_row(double* p, const T* v) {
-#pragma unroll
-  for (int m = 0; m < 4; ++m) reinterpret_cast<double2*>(p)[m] = make_double2((double)v[2 * m], (double)v[2 * m + 1]);
 }
 template <typename T>
 __device__ __forceinline__ void store_row(__nv_bfloat16* p, const T* v) {
@@ -1740,31 +1731,41 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
   // level storage: T, or BF16 for levels 1 .. bf16_hi-1 (FP32 solvers with coarse_bf16)
   using BF = __nv_bfloat16;
   auto bf = [&](int l) { return std::is_same<T, float>::value && l >= 1 && l < S->bf16_hi; };
-  const bool split = D == 3 && S->rs;  // the per-level levels are stored by colour
+  constexpr bool kCanSplit = D == 3 && std::is_same<T, float>::value;
+  const bool split = kCanSplit && S->rs;  // the per-level levels are stored by colour
   auto rl = [&](int l) { return l == 0 && split ? (T*)S->rs : r[l]; };
   auto sweep = [&](int l, int phase) {
     const Shape sh = S->lv[l];
-    if (split) {
-      const Rows w = rows_of(sh, 128);
-      if (bf(l)) launch_pdl(k_smooth_split<T, BF, false>, (unsigned)w.items, 128, 0, s, sh, w, (const BF*)S->r[l], (BF*)S->z[l], phase, (BF*)nullptr, nullptr, S->st);
-      else launch_pdl(k_smooth_split<T, T, false>, (unsigned)w.items, 128, 0, s, sh, w, (const T*)rl(l), z[l], phase, (T*)nullptr, nullptr, S->st);
-    } else if (bf(l)) launch_pdl(k_smooth_pair<T, D, BF>, pair_grid(sh), pblk, 0, s, sh, (const BF*)S->r[l], (BF*)S->z[l], phase, S->st);
+    if constexpr (kCanSplit) {
+      if (split) {
+        const Rows w = rows_of(sh, 128);
+        if (bf(l)) launch_pdl(k_smooth_split<T, BF, false>, (unsigned)w.items, 128, 0, s, sh, w, (const BF*)S->r[l], (BF*)S->z[l], phase, (BF*)nullptr, nullptr, S->st);
+        else launch_pdl(k_smooth_split<T, T, false>, (unsigned)w.items, 128, 0, s, sh, w, (const T*)rl(l), z[l], phase, (T*)nullptr, nullptr, S->st);
+        return;
+      }
+    }
+    if (bf(l)) launch_pdl(k_smooth_pair<T, D, BF>, pair_grid(sh), pblk, 0, s, sh, (const BF*)S->r[l], (BF*)S->z[l], phase, S->st);
     else launch_pdl(k_smooth_pair<T, D>, pair_grid(sh), pblk, 0, s, sh, (const T*)r[l], z[l], phase, S->st);
+  };
+  auto first_sweep = [&](int l) {
+    const Shape sh = S->lv[l];
+    const int rec = l == 0 && recenter ? 1 : 0;
+    if constexpr (kCanSplit) {
+      if (split) {
+        const Rows w = rows_of(sh, 128);
+        if (bf(l)) launch_pdl(k_first_split<T, BF>, (unsigned)w.items, 128, 0, s, sh, w, (BF*)nullptr, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
+        else launch_pdl(k_first_split<T, T>, (unsigned)w.items, 128, 0, s, sh, w, l == 0 ? r[0] : (T*)nullptr, rl(l), z[l], S->st, rec);
+        return;
+      }
+    }
+    if (bf(l)) launch_pdl(k_smooth_first_pair<T, D, BF>, pair_grid(sh), pblk, 0, s, sh, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
+    else launch_pdl(k_smooth_first_pair<T, D>, pair_grid(sh), pblk, 0, s, sh, r[l], z[l], S->st, rec);
   };
   for (int l = 0; l < lc; ++l) {
     const Shape sh = S->lv[l];
-    const dim3 pg = pair_grid(sh);
     for (int it = 0; it < P.pre_post; ++it) {
-      if (it == 0 && split) {
-        const Rows w = rows_of(sh, 128);
-        if (bf(l)) launch_pdl(k_first_split<T, BF>, (unsigned)w.items, 128, 0, s, sh, w, (BF*)nullptr, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
-        else launch_pdl(k_first_split<T, T>, (unsigned)w.items, 128, 0, s, sh, w, l == 0 ? r[0] : (T*)nullptr, rl(l), z[l], S->st, l == 0 && recenter ? 1 : 0);
-      } else if (it == 0) {
-        if (bf(l)) launch_pdl(k_smooth_first_pair<T, D, BF>, pg, pblk, 0, s, sh, (BF*)S->r[l], (BF*)S->z[l], S->st, 0);
-        else launch_pdl(k_smooth_first_pair<T, D>, pg, pblk, 0, s, sh, r[l], z[l], S->st, l == 0 && recenter ? 1 : 0);
-      } else {
-        sweep(l, 0);
-      }
+      if (it == 0) first_sweep(l);
+      else sweep(l, 0);
       sweep(l, 1);
     }
     const Shape sc = S->lv[l + 1];
@@ -1775,8 +1776,9 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
         const bool vec = two_aligned(rf, sizeof(SF), sh) && two_aligned(zf, sizeof(SF), sh);
         const int out_split = split && l + 1 < lc;
         using SC = std::remove_pointer_t<decltype(rc)>;
-        launch_pdl(split ? k_restrict_walk<T, SF, SC, kSplit> : (vec ? k_restrict_walk<T, SF, SC, kVec> : k_restrict_walk<T, SF, SC, kOne>),
-                   (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, (const SF*)rf, (const SF*)zf, rc, out_split, (const DevState*)S->st);
+        auto k = vec ? k_restrict_walk<T, SF, SC, kVec> : k_restrict_walk<T, SF, SC, kOne>;
+        if constexpr (kCanSplit) k = split ? k_restrict_walk<T, SF, SC, kSplit> : k;
+        launch_pdl(k, (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, (const SF*)rf, (const SF*)zf, rc, out_split, (const DevState*)S->st);
       };
       if (bf(l) && bf(l + 1)) go((BF*)S->r[l], (BF*)S->z[l], (BF*)S->r[l + 1]);
       else if (bf(l)) go((BF*)S->r[l], (BF*)S->z[l], r[l + 1]);
@@ -1829,8 +1831,9 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
         using SF = std::remove_pointer_t<decltype(zf)>;
         using SC = std::remove_pointer_t<decltype(zc)>;
         const bool vec = two_aligned(zf, sizeof(SF), sh);
-        launch_pdl(split ? k_prolong_walk<T, SF, SC, kSplit> : (vec ? k_prolong_walk<T, SF, SC, kVec> : k_prolong_walk<T, SF, SC, kOne>),
-                   (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, zf, (const SC*)zc, (int)(split && l + 1 < lc),
+        auto k = vec ? k_prolong_walk<T, SF, SC, kVec> : k_prolong_walk<T, SF, SC, kOne>;
+        if constexpr (kCanSplit) k = split ? k_prolong_walk<T, SF, SC, kSplit> : k;
+        launch_pdl(k, (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, zf, (const SC*)zc, (int)(split && l + 1 < lc),
                    (const DevState*)S->st);
       };
       if (bf(l) && bf(l + 1)) go((BF*)S->z[l], (BF*)S->z[l + 1]);
@@ -1851,11 +1854,15 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
     for (int it = 0; it < P.pre_post; ++it) {
       sweep(l, 1);
       const bool end = l == 0 && it == P.pre_post - 1, last = dot_last && end;
-      if (end && split) {
-        const Rows w = rows_of(sh, 256);
-        launch_pdl(k_smooth_split<T, T, true>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), 256, 0, s, sh, w,
-                   (const T*)S->rs, z[0], 0, (T*)S->Ap, S->part, S->st);
-      } else if (!last) {
+      if constexpr (kCanSplit) {
+        if (end && split) {
+          const Rows w = rows_of(sh, 256);
+          launch_pdl(k_smooth_split<T, T, true>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), 256, 0, s, sh, w,
+                     (const T*)S->rs, z[0], 0, (T*)S->Ap, S->part, S->st);
+          continue;
+        }
+      }
+      if (!last) {
         sweep(l, 0);
       } else if constexpr (D == 3) {
         const Walk w = walk_pairs(sh, kRedBlocks);
@@ -2154,10 +2161,10 @@ int fm_mgpcg_create(const fm_grid* g, int dtype, const fm_mg_params* params, fm_
     ok = ok && cudaMalloc(&S->z[l], e * S->lv[l].size()) == cudaSuccess;
   }
   const long n0 = S->lv[0].size();
-  // 3D levels of 16 n cells a row are stored by colour: a second residual, in x's allocation; without the memory
-  // for it the levels stay in natural order
+  // levels of 16 n cells a row of a large 3D FP32 solver are stored by colour: a second residual, in x's
+  // allocation; without the memory for it the levels stay in natural order
   const int fine = S->lc > 0 ? S->lc : S->L - 1;
-  bool split = g->dim == 3 && !S->pcg_nc && P.pre_post > 0 && fine > 0;
+  bool split = g->dim == 3 && dtype == FM_F32 && n0 >= kSplitCells && !S->pcg_nc && fine > 0;
   for (int l = 0; l < fine; ++l) split = split && split_fits(S->lv[l]);
   if (split && ok) {
     const size_t xb = (es * n0 + 255) / 256 * 256;
