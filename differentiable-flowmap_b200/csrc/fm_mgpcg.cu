@@ -864,6 +864,11 @@ struct Walk {
   int tk, tj, planes, items;
 };
 constexpr int kWalkBX = 32, kWalkBY = 8, kWalkBlocks = 148 * 7;
+// The two kernels with an inner product walk in FP32 only: in FP64 the grid-stride ones are faster
+// (144^3, us, walking / not: last half-sweep 30.1 / 23.7, A p 28.0 / 19.0; 128^3 18.4 / 17.7 and 12.6 / 10.6;
+// 40^3 4.9 / 4.3 and 3.8 / 3.4).
+template <typename T, int D>
+constexpr bool kWalkDots = D == 3 && std::is_same<T, float>::value;
 // over n0 planes, n1 rows, nk columns of the threads, in at most `most` items where
 // stretches of whole columns allow
 inline Walk walk_of(int n0, int n1, int nk, int most) {
@@ -1864,7 +1869,7 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
       }
       if (!last) {
         sweep(l, 0);
-      } else if constexpr (D == 3) {
+      } else if constexpr (kWalkDots<T, D>) {
         const Walk w = walk_pairs(sh, kRedBlocks);
         launch_pdl(k_smooth_dot_walk<T>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock, 0, s, sh, w,
                    (const T*)r[l], z[l], 0, S->part, S->st);
@@ -1885,7 +1890,7 @@ template <typename T, int D>
 static void launch_step(fm_mgpcg* S, cudaStream_t s) {
   const Shape s0 = S->lv[0];
   const long n = s0.size();
-  if constexpr (D == 3) {
+  if constexpr (kWalkDots<T, D>) {
     const Walk w = walk_pairs(s0, kRedBlocks);
     const bool vec = two_aligned(S->p, sizeof(T), s0) && two_aligned(S->Ap, sizeof(T), s0);
     launch_pdl(vec ? k_Ap_walk<T, kVec> : k_Ap_walk<T, kOne>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock,
