@@ -34,6 +34,7 @@
 // the face's high side wins.  mask_passive gives a solid cell the mean of its
 // fluid 3^dim neighbours (lexicographic offset order) or 0.
 #include <math.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <stdlib.h>
 
@@ -163,25 +164,33 @@ __global__ void k_mask0(long n, const float* __restrict__ mask, uint8_t* __restr
     fl[q] = mask[q] > 0.f ? 0 : 1;
 }
 
+// Flags of a level as the packing below reads them: stored, or (the level being
+// made) from the flags of the level above it: fluid where any child is.
 template <int D>
-__global__ void k_downsample(Shape sf, const uint8_t* __restrict__ ff, Shape sc, uint8_t* __restrict__ fc) {
-  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < sc.size(); q += (long)gridDim.x * blockDim.x) {
-    int I[3];
-    idx3(sc, q, I);
+struct Stored {
+  const uint8_t* fl;
+  __device__ __forceinline__ bool operator()(const Shape& s, const int* I) const { return fl[s.idx(I[0], I[1], I[2])]; }
+};
+template <int D>
+struct FromFine {
+  Shape sf;
+  const uint8_t* ff;
+  __device__ __forceinline__ bool operator()(const Shape&, const int* I) const {
     uint8_t any = 0;
     for (int d0 = 0; d0 < 2; ++d0)
       for (int d1 = 0; d1 < 2; ++d1)
-        for (int d2 = 0; d2 < (D == 3 ? 2 : 1); ++d2) any |= ff[sf.idx(2 * I[0] + d0, 2 * I[1] + d1, D == 3 ? 2 * I[2] + d2 : 0)];
-    fc[q] = any;
+        for (int d2 = 0; d2 < (D == 3 ? 2 : 1); ++d2)
+          any |= ff[sf.idx(2 * I[0] + d0, 2 * I[1] + d1, D == 3 ? 2 * I[2] + d2 : 0)];
+    return any;
   }
-}
+};
 
 // The obstacle mask of a level as the cluster solve reads it: one word per pair
 // of cells (2m, 2m + 1) of a row, holding per colour c at bit 8c the in-domain
 // fluid neighbours (+i -i +j -j +k -k; in 2D the last two are +j -j) and, at
 // bit 6, whether the cell is fluid (fm_mg_cluster.cuh).
-template <int D>
-__global__ void k_pack_mask(Shape s, const uint8_t* __restrict__ fl, uint16_t* __restrict__ out) {
+template <int D, typename Flags>
+__device__ __forceinline__ void pack_mask(const Shape& s, const Flags& fluid, uint16_t* __restrict__ out) {
   const int nin = D == 3 ? s.s2 : s.s1, M = (nin + 1) / 2;
   const long rows = (long)s.s0 * (D == 3 ? s.s1 : 1);
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < rows * M; e += (long)gridDim.x * blockDim.x) {
@@ -191,21 +200,39 @@ __global__ void k_pack_mask(Shape s, const uint8_t* __restrict__ fl, uint16_t* _
     for (int h = 0; h < 2; ++h) {
       const int k = 2 * m + h;
       if (k >= nin) continue;
-      const long q = row * nin + k;
-      if (!fl[q]) continue;
       int I[3];
-      idx3(s, q, I);
+      idx3(s, row * nin + k, I);
+      if (!fluid(s, I)) continue;
       unsigned b = 64;
       for (int a = 0; a < D; ++a) {
-        const long st = stride_of(s, a);
-        const int sh = a == D - 1 ? 4 : 2 * a;
-        if (I[a] < axis_len(s, a) - 1 && fl[q + st]) b |= 1u << sh;
-        if (I[a] > 0 && fl[q - st]) b |= 2u << sh;
+        const int sh = a == D - 1 ? 4 : 2 * a, x = I[a];
+        I[a] = x + 1;
+        if (x < axis_len(s, a) - 1 && fluid(s, I)) b |= 1u << sh;
+        I[a] = x - 1;
+        if (x > 0 && fluid(s, I)) b |= 2u << sh;
+        I[a] = x;
       }
       w |= b << (8 * ((I[0] + I[1] + I[2]) & 1));
     }
     out[e] = (uint16_t)w;
   }
+}
+
+// The flags of a level from those of the level above it, and, for a cluster solve, the
+// packed masks of that one (mf) and, on the coarsest level, of this one (mc): a launch per
+// level as without them, since the launches are all that this costs (256^2, five levels:
+// 28 us, 46 us with a launch more per level).
+template <int D>
+__global__ void k_downsample(Shape sf, const uint8_t* __restrict__ ff, Shape sc, uint8_t* __restrict__ fc,
+                             uint16_t* __restrict__ mf, uint16_t* __restrict__ mc) {
+  const FromFine<D> coarse{sf, ff};
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < sc.size(); q += (long)gridDim.x * blockDim.x) {
+    int I[3];
+    idx3(sc, q, I);
+    fc[q] = coarse(sc, I);
+  }
+  if (mf) pack_mask<D>(sf, Stored<D>{ff}, mf);
+  if (mc) pack_mask<D>(sc, coarse, mc);
 }
 
 // z = (r + sum) / n with div_nd (rounded as the IEEE quotient)
@@ -500,11 +527,11 @@ __global__ void k_update_p(long n, T* __restrict__ p, const T* __restrict__ z, c
 }
 
 template <typename T>
-__global__ void k_init(long n, const T* __restrict__ b, T k, T* __restrict__ r, T* __restrict__ x, T* __restrict__ p) {
+__global__ void k_init(long n, const T* __restrict__ b, T* __restrict__ r, T* __restrict__ x, T* __restrict__ p) {
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-    r[q] = b[q] * k;
+    r[q] = b[q];
     x[q] = (T)0;
-    p[q] = (T)0;
+    if (p) p[q] = (T)0;
   }
 }
 
@@ -544,7 +571,7 @@ __global__ void k_project_front(fm_grid g, const T* __restrict__ ux, const T* __
     }
     r[q] = acc * (T)-1;
     x[q] = (T)0;
-    p[q] = (T)0;
+    if (p) p[q] = (T)0;
   }
 }
 
@@ -969,7 +996,7 @@ int project(fm_solid* S, void* const* u, void* p_out, cudaStream_t s, int* iters
 template <typename T, int D>
 int solve_rhs(fm_solid* S, const void* b, void* x, cudaStream_t s, int* iters, double* rtr) {
   const long n = S->sh[0].size();
-  launch(k_init<T>, blocks_for(n), kThreads, 0, s, n, (const T*)b, (T)1, (T*)S->r[0], (T*)S->x, (T*)S->p);
+  launch(k_init<T>, blocks_for(n), kThreads, 0, s, n, (const T*)b, (T*)S->r[0], (T*)S->x, (T*)S->p);
   return solve<T, D>(S, x, s, iters, rtr);
 }
 
@@ -979,14 +1006,18 @@ int solve_rhs(fm_solid* S, const void* b, void* x, cudaStream_t s, int* iters, d
 namespace fm {
 namespace solid {
 
-// The packed masks of every level, from the fluid flags (cluster solves only).
-static void pack_masks(fm_solid* S, cudaStream_t s) {
-  if (!S->pcg_nc) return;
-  for (int l = 0; l < S->levels; ++l) {
-    const unsigned nb = blocks_for(S->sh[l].size());
-    if (S->dim == 2) launch(k_pack_mask<2>, nb, kThreads, 0, s, S->sh[l], (const uint8_t*)S->fl[l], S->msk[l]);
-    else launch(k_pack_mask<3>, nb, kThreads, 0, s, S->sh[l], (const uint8_t*)S->fl[l], S->msk[l]);
-  }
+// The flags of the levels below the finest, and every level's packed mask.
+template <int D>
+static void refresh_masks(fm_solid* S, cudaStream_t s) {
+  const bool packed = S->pcg_nc != 0;
+  for (int l = 1; l < S->levels; ++l)
+    launch(k_downsample<D>, blocks_for(S->sh[packed ? l - 1 : l].size()), kThreads, 0, s, S->sh[l - 1],
+           (const uint8_t*)S->fl[l - 1], S->sh[l], S->fl[l], packed ? S->msk[l - 1] : nullptr,
+           packed && l == S->levels - 1 ? S->msk[l] : nullptr);
+}
+static void refresh_masks(fm_solid* S, cudaStream_t s) {
+  if (S->dim == 2) refresh_masks<2>(S, s);
+  else refresh_masks<3>(S, s);
 }
 
 template <typename T, int D>
@@ -1024,12 +1055,9 @@ int fm_solid_destroy(fm_solid* S) {
   cudaFree(S->x);
   cudaFree(S->p);
   cudaFree(S->Ap);
-  cudaFree(S->part);
   cudaFree(S->d_pcg);
-  cudaFree(S->st);
-  cudaFree(S->stats);
-  if (S->st_host) cudaFreeHost(S->st_host);
-  if (S->stats_host) cudaFreeHost(S->stats_host);
+  cudaFree(S->st);  // with the statistics and the partial sums
+  if (S->st_host) cudaFreeHost(S->st_host);  // with the statistics
   if (S->chunk) cudaGraphExecDestroy(S->chunk);
   if (S->loop) cudaGraphExecDestroy(S->loop);
   if (S->cap) cudaStreamDestroy(S->cap);
@@ -1042,15 +1070,7 @@ int fm_solid_set_mask(fm_solid* S, const float* mask, void* stream) {
   if (!S || !mask) return FM_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   fm::launch(k_mask0, blocks_for(S->sh[0].size()), kThreads, 0, s, S->sh[0].size(), mask, S->fl[0]);
-  for (int l = 1; l < S->levels; ++l) {
-    if (S->dim == 2)
-      fm::launch(k_downsample<2>, blocks_for(S->sh[l].size()), kThreads, 0, s, S->sh[l - 1], (const uint8_t*)S->fl[l - 1],
-                 S->sh[l], S->fl[l]);
-    else
-      fm::launch(k_downsample<3>, blocks_for(S->sh[l].size()), kThreads, 0, s, S->sh[l - 1], (const uint8_t*)S->fl[l - 1],
-                 S->sh[l], S->fl[l]);
-  }
-  pack_masks(S, s);
+  refresh_masks(S, s);
   return fm::check_cuda();
 }
 
@@ -1082,20 +1102,27 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
     ok = ok && cudaMalloc(&S->z[l], sh.size() * es) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&S->fl[l], sh.size()) == cudaSuccess;
   }
-  const long n = S->sh[0].size();
-  ok = ok && cudaMalloc(&S->x, n * es) == cudaSuccess && cudaMalloc(&S->p, n * es) == cudaSuccess &&
-       cudaMalloc(&S->Ap, n * es) == cudaSuccess &&
-       cudaMalloc((void**)&S->part, solid::kRedBlocks * sizeof(double)) == cudaSuccess &&
-       cudaMalloc((void**)&S->st, sizeof(solid::State)) == cudaSuccess &&
-       cudaMallocHost((void**)&S->st_host, sizeof(solid::State)) == cudaSuccess &&
-       cudaMalloc((void**)&S->stats, sizeof(solid::Stats)) == cudaSuccess &&
-       cudaMallocHost((void**)&S->stats_host, sizeof(solid::Stats)) == cudaSuccess &&
-       cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) == cudaSuccess;
-  if (ok) ok = cudaMemset(S->stats, 0, sizeof(solid::Stats)) == cudaSuccess;
   if (ok) {
     if (dtype == FM_F32) ok = g->dim == 2 ? solid::plan_cluster<float, 2>(S) : solid::plan_cluster<float, 3>(S);
     else ok = g->dim == 2 ? solid::plan_cluster<double, 2>(S) : solid::plan_cluster<double, 3>(S);
   }
+  const long n = S->sh[0].size();
+  ok = ok && cudaMalloc(&S->x, n * es) == cudaSuccess;
+  if (!S->pcg_nc)  // a cluster solve keeps p and A p in shared memory and records no graphs
+    ok = ok && cudaMalloc(&S->p, n * es) == cudaSuccess && cudaMalloc(&S->Ap, n * es) == cudaSuccess &&
+         cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) == cudaSuccess;
+  // state, statistics and partial sums in one allocation, their host copies in another
+  struct Small {
+    solid::State st;
+    solid::Stats stats;
+    double part[solid::kRedBlocks];
+  };
+  Small *small = nullptr, *host = nullptr;
+  ok = ok && cudaMalloc((void**)&small, sizeof(Small)) == cudaSuccess;
+  if (ok) S->st = &small->st, S->stats = &small->stats, S->part = small->part;
+  ok = ok && cudaMallocHost((void**)&host, offsetof(Small, part)) == cudaSuccess;
+  if (ok) S->st_host = &host->st, S->stats_host = &host->stats;
+  if (ok) ok = cudaMemset(S->stats, 0, sizeof(solid::Stats)) == cudaSuccess;
   if (!ok) {
     fm_solid_destroy(S);
     return FM_ERR_CUDA;
@@ -1115,8 +1142,8 @@ int fm_solid_create(const fm_grid* g, int dtype, const fm_mg_params* params, con
       return ms;
     }
   } else {
-    for (int l = 0; l < P.levels; ++l) cudaMemset(S->fl[l], 1, S->sh[l].size());
-    solid::pack_masks(S, nullptr);
+    cudaMemset(S->fl[0], 1, S->sh[0].size());
+    solid::refresh_masks(S, nullptr);
     cudaStreamSynchronize(nullptr);  // the first solve may come on a stream that the default one does not order
   }
   *out = S;
