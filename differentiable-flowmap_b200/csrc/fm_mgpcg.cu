@@ -803,14 +803,13 @@ __global__ void __launch_bounds__(kRedThreads) k_smooth(Shape s, const T* __rest
   if (DOT) block_reduce2(acc, 0.0, part + 2 * blockIdx.x);
 }
 
-// restrict(l) (3D/mgpcg.py:157-163) as a gather over the 2^D children.
+// restrict(l) (3D/mgpcg.py:157-163) as a gather over the 4 children, 2D (3D: k_restrict_walk).
 // SF / SC: storage types of the fine and the coarse level.
-template <typename T, int D, typename SF = T, typename SC = T>
+template <typename T, typename SF = T, typename SC = T>
 __global__ void k_restrict(Shape sf, Shape sc, const SF* __restrict__ rf, const SF* __restrict__ zf,
                            SC* __restrict__ rc, const DevState* st) {
   pdl_begin();
   if (st->done) return;
-  const T scale = (T)1.0 / (T)(D - 1.0);
   FM_GRID_STRIDE(q, sc.size()) {
     int I, J, K;
     unflatten(sc, q, I, J, K);
@@ -818,29 +817,26 @@ __global__ void k_restrict(Shape sf, Shape sc, const SF* __restrict__ rf, const 
 #pragma unroll
     for (int di = 0; di < 2; ++di)
 #pragma unroll
-      for (int dj = 0; dj < 2; ++dj)
-#pragma unroll
-        for (int dk = 0; dk < (D == 3 ? 2 : 1); ++dk) {
-          const int i = 2 * I + di, j = 2 * J + dj, k = D == 3 ? 2 * K + dk : 0;
-          const long f = sf.idx(i, j, k);
-          T diag;
-          const T nb = nb_sum_s<T, D, SF>(zf, sf, i, j, k, diag);
-          const T res = rn_sub((T)to_c(rf[f]), rn_sub(rn_mul(diag, (T)to_c(zf[f])), nb));
-          acc = rn_add(acc, rn_mul(res, scale));
-        }
+      for (int dj = 0; dj < 2; ++dj) {
+        const int i = 2 * I + di, j = 2 * J + dj;
+        const long f = sf.idx(i, j, 0);
+        T diag;
+        const T nb = nb_sum_s<T, 2, SF>(zf, sf, i, j, 0, diag);
+        acc = rn_add(acc, rn_sub((T)to_c(rf[f]), rn_sub(rn_mul(diag, (T)to_c(zf[f])), nb)));  // scale 1 / (D - 1)
+      }
     rc[q] = to_s<SC>(acc);
   }
 }
 
-// prolongate(l) (3D/mgpcg.py:165-168)
-template <typename T, int D, typename SF = T, typename SC = T>
+// prolongate(l) (3D/mgpcg.py:165-168), 2D (3D: k_prolong_walk)
+template <typename T, typename SF = T, typename SC = T>
 __global__ void k_prolong(Shape sf, Shape sc, SF* __restrict__ zf, const SC* __restrict__ zc, const DevState* st) {
   pdl_begin();
   if (st->done) return;
   FM_GRID_STRIDE(q, sf.size()) {
     int i, j, k;
     unflatten(sf, q, i, j, k);
-    zf[q] = to_s<SF>((T)to_c(zf[q]) + (T)to_c(zc[sc.idx(i >> 1, j >> 1, D == 3 ? (k >> 1) : 0)]));
+    zf[q] = to_s<SF>((T)to_c(zf[q]) + (T)to_c(zc[sc.idx(i >> 1, j >> 1, 0)]));
   }
 }
 
@@ -892,16 +888,20 @@ __device__ __forceinline__ void walk_item(const Walk& w, int it, int n0, int& i0
   i1 = min(i0 + w.planes, n0);
 }
 
-// How a pair of cells of a row is stored: one by one, by one aligned load (an even row
-// length and an aligned array), or by colour (below).
-enum { kOne = 0, kVec = 1, kSplit = 2 };
-// The pair at p; ha / hb: its cells exist (0 otherwise); oa: kSplit, the offset of
-// the first one's colour (0 or h), p then points at the pair in the first colour.
+// How a pair of cells of a row is stored: side by side, read by one aligned load (rows of
+// every level but the coarsest have an even length: creation asks for cell counts that are
+// multiples of 2^(levels - 1)), or by colour (below).
+enum { kVec = 0, kSplit = 1 };
+// The pair at p, zeros where `on` is false; oa: kSplit, the offset of the first one's
+// colour (0 or h), p then points at the pair in the first colour.
 template <int MODE, typename T, typename S>
-__device__ __forceinline__ void load_two(const S* p, bool ha, bool hb, T& a, T& b, int oa = 0, int h = 0) {
-  if constexpr (MODE == kVec) {
+__device__ __forceinline__ void load_two(const S* p, bool on, T& a, T& b, int oa = 0, int h = 0) {
+  if constexpr (MODE == kSplit) {
+    a = on ? (T)to_c(p[oa]) : (T)0;
+    b = on ? (T)to_c(p[h - oa]) : (T)0;
+  } else {
     a = b = (T)0;
-    if (hb) {
+    if (on) {
       if constexpr (std::is_same<S, __nv_bfloat16>::value) {
         const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(p);
         a = (T)__low2float(v), b = (T)__high2float(v);
@@ -911,19 +911,12 @@ __device__ __forceinline__ void load_two(const S* p, bool ha, bool hb, T& a, T& 
         a = (T)v.x, b = (T)v.y;
       }
     }
-  } else {
-    a = ha ? (T)to_c(p[MODE == kSplit ? oa : 0]) : (T)0;
-    b = hb ? (T)to_c(p[MODE == kSplit ? h - oa : 1]) : (T)0;
   }
 }
 // neighbours of a cell within its plane
 __device__ __forceinline__ int plane_nd(const Shape& s, int j, int k) {
   return 6 - (j == 0) - (j == s.s1 - 1) - (k == 0) - (k == s.s2 - 1);
 }
-inline bool two_aligned(const void* p, size_t elem, const Shape& s) {
-  return s.s2 % 2 == 0 && (uintptr_t)p % (2 * elem) == 0;
-}
-
 // smooth(l, phase) (3D/mgpcg.py:170-177), only the cells of colour `phase`, and
 // the partial sums of z.r over all cells.  The other colour's cell of a
 // pair is the +-i neighbour of the updated cells in the planes beside, and a +-k
@@ -1022,7 +1015,7 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_smooth_dot_walk(Shape s, W
 }
 
 // Ap = A p and the partial sums of p.Ap
-template <typename T, int MODE>
+template <typename T>
 __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_Ap_walk(Shape s, Walk w, const T* __restrict__ p,
                                                              T* __restrict__ Ap, double* __restrict__ part,
                                                              const DevState* st) {
@@ -1037,9 +1030,8 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_Ap_walk(Shape s, Walk w, c
     walk_item(w, it, s.s0, i0, i1, j, m);
     if (j >= s.s1) continue;  // the whole warp
     const int k0 = 2 * m;
-    const bool ha = k0 < s.s2, hb = k0 + 1 < s.s2;
-    const bool pa = ha && j < s.s1 - 1, pb = hb && j < s.s1 - 1, la = ha && j > 0, lb = hb && j > 0;
-    const bool edge = (lane == 0 && ha && k0 > 0) || (lane == 31 && k0 + 2 < s.s2);
+    const bool on = k0 < s.s2, jp = on && j < s.s1 - 1, jm = on && j > 0;
+    const bool edge = (lane == 0 && on && k0 > 0) || (lane == 31 && k0 + 2 < s.s2);
     const int eo = lane == 0 ? -1 : 2;
     const T nda = (T)plane_nd(s, j, k0), ndb = (T)plane_nd(s, j, k0 + 1);
     const long q = ((long)i0 * s.s1 + j) * s.s2 + k0;
@@ -1050,14 +1042,14 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_Ap_walk(Shape s, Walk w, c
     };
     const auto fetch = [&](const T* x, bool in, bool whole) {
       Plane v;
-      load_two<MODE>(x, in && ha, in && hb, v.a, v.b);
-      load_two<MODE>(x + sj, whole && pa, whole && pb, v.pa, v.pb);
-      load_two<MODE>(x - sj, whole && la, whole && lb, v.ma, v.mb);
+      load_two<kVec>(x, in && on, v.a, v.b);
+      load_two<kVec>(x + sj, whole && jp, v.pa, v.pb);
+      load_two<kVec>(x - sj, whole && jm, v.ma, v.mb);
       v.far = whole && edge ? x[eo] : (T)0;
       return v;
     };
     T ma, mb;
-    load_two<MODE>(pp - si, i0 > 0 && ha, i0 > 0 && hb, ma, mb);
+    load_two<kVec>(pp - si, i0 > 0 && on, ma, mb);
     Plane c = fetch(pp, true, true);
 #pragma unroll 2
     for (int i = i0; i < i1; ++i) {
@@ -1069,13 +1061,8 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_Ap_walk(Shape s, Walk w, c
       nb += n.b, nb += mb, nb += c.pb, nb += c.mb, nb += right, nb += c.a;
       const T wall = (T)((i == 0) + (i == s.s0 - 1));
       const T ra = rn_sub(rn_mul(nda - wall, c.a), na), rb = rn_sub(rn_mul(ndb - wall, c.b), nb);
-      if constexpr (MODE == kVec) {
-        using V = std::conditional_t<std::is_same<T, float>::value, float2, double2>;
-        if (hb) *reinterpret_cast<V*>(ap) = V{ra, rb};
-      } else {
-        if (ha) ap[0] = ra;
-        if (hb) ap[1] = rb;
-      }
+      using V = std::conditional_t<std::is_same<T, float>::value, float2, double2>;
+      if (on) *reinterpret_cast<V*>(ap) = V{ra, rb};
       acc += (double)c.a * (double)ra;  // a missing cell is 0
       acc += (double)c.b * (double)rb;
       ma = c.a, mb = c.b;
@@ -1111,7 +1098,7 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_restrict_walk(Shape sf, Sh
     const int k0 = 2 * K, j0 = 2 * J;
     const bool jl = on && j0 > 0, jh = on && j0 + 2 < sf.s1;
     const bool el = on && lane == 0 && k0 > 0;
-    const bool er = on && k0 + 2 < sf.s2 && (lane == 31 || K + 1 >= sc.s2);  // a last odd cell has no pair
+    const bool er = on && lane == 31 && k0 + 2 < sf.s2;
     T nd[2][2];
 #pragma unroll
     for (int d = 0; d < 2; ++d) nd[d][0] = (T)plane_nd(sf, j0 + d, k0), nd[d][1] = (T)plane_nd(sf, j0 + d, k0 + 1);
@@ -1123,8 +1110,8 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_restrict_walk(Shape sf, Sh
     T ma[2], mb[2], ca[2], cb[2];
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
-      load_two<MODE>(zp - si + d * sj, on && I0 > 0, on && I0 > 0, ma[d], mb[d], d ? 0 : h, h);
-      load_two<MODE>(zp + d * sj, on, on, ca[d], cb[d], d ? h : 0, h);
+      load_two<MODE>(zp - si + d * sj, on && I0 > 0, ma[d], mb[d], d ? 0 : h, h);
+      load_two<MODE>(zp + d * sj, on, ca[d], cb[d], d ? h : 0, h);
     }
     for (int I = I0; I < I1; ++I) {
       T acc = (T)0;
@@ -1136,19 +1123,19 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_restrict_walk(Shape sf, Sh
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
           const int oa = ((d + di) & 1) ? h : 0;  // the first cell's colour
-          load_two<MODE>(zp + si + d * sj, up, up, na[d], nb[d], h - oa, h);
-          load_two<MODE>(rp + d * sj, on, on, ra[d], rb[d], oa, h);
+          load_two<MODE>(zp + si + d * sj, up, na[d], nb[d], h - oa, h);
+          load_two<MODE>(rp + d * sj, on, ra[d], rb[d], oa, h);
           eL[d] = el ? (T)to_c(zp[d * sj + (MODE == kSplit ? h - oa - 1 : -1)]) : (T)0;
           eR[d] = er ? (T)to_c(zp[d * sj + (MODE == kSplit ? oa + 1 : 2)]) : (T)0;
         }
-        load_two<MODE>(zp - sj, jl, jl, xa[0], xb[0], di ? 0 : h, h);
-        load_two<MODE>(zp + 2 * sj, jh, jh, xa[1], xb[1], di ? h : 0, h);
+        load_two<MODE>(zp - sj, jl, xa[0], xb[0], di ? 0 : h, h);
+        load_two<MODE>(zp + 2 * sj, jh, xa[1], xb[1], di ? h : 0, h);
         const T wall = (T)((i == 0) + (i == sf.s0 - 1));
 #pragma unroll
         for (int d = 0; d < 2; ++d) {  // row j0 + d
           T left = __shfl_up_sync(all, cb[d], 1), right = __shfl_down_sync(all, ca[d], 1);
           if (lane == 0) left = eL[d];
-          if (lane == 31 || er) right = eR[d];
+          if (lane == 31) right = eR[d];
           const T pa = d == 0 ? ca[1] : xa[1], pb = d == 0 ? cb[1] : xb[1];  // +j
           const T la = d == 0 ? xa[0] : ca[0], lb = d == 0 ? xb[0] : cb[0];  // -j
           T sa = (T)0, sb = (T)0;
@@ -1184,7 +1171,6 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_prolong_walk(Shape sf, Sha
     walk_item(w, it, sf.s0, i0, i1, j, m);
     const int k0 = 2 * m;
     if (j >= sf.s1 || k0 >= sf.s2) continue;
-    const bool hb = k0 + 1 < sf.s2;
     unsigned q = ((unsigned)i0 * sf.s1 + j) * sf.s2 + (MODE == kSplit ? m : k0);
     const SC* const zcol = zc + (j >> 1) * (unsigned)sc.s2;
     const int h = sf.s2 / 2;
@@ -1195,9 +1181,9 @@ __global__ void __launch_bounds__(kWalkBX* kWalkBY) k_prolong_walk(Shape sf, Sha
       const T c = (T)to_c(zcol[I * sci + at]);
       const int oa = MODE == kSplit && ((i + j) & 1) ? h : 0, ob = MODE == kSplit ? h - oa : 1;
       T a, b;
-      load_two<MODE>(zf + q, true, hb, a, b, oa, h);
+      load_two<MODE>(zf + q, true, a, b, oa, h);
       zf[q + oa] = to_s<SF>(a + c);
-      if (hb) zf[q + ob] = to_s<SF>(b + c);
+      zf[q + ob] = to_s<SF>(b + c);
     }
   }
 }
@@ -1778,10 +1764,9 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
       const Walk w = walk_of(sc.s0, sc.s1, sc.s2, kWalkBlocks);
       auto go = [&](auto* rf, auto* zf, auto* rc) {
         using SF = std::remove_pointer_t<decltype(rf)>;
-        const bool vec = two_aligned(rf, sizeof(SF), sh) && two_aligned(zf, sizeof(SF), sh);
         const int out_split = split && l + 1 < lc;
         using SC = std::remove_pointer_t<decltype(rc)>;
-        auto k = vec ? k_restrict_walk<T, SF, SC, kVec> : k_restrict_walk<T, SF, SC, kOne>;
+        auto k = k_restrict_walk<T, SF, SC, kVec>;
         if constexpr (kCanSplit) k = split ? k_restrict_walk<T, SF, SC, kSplit> : k;
         launch_pdl(k, (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, (const SF*)rf, (const SF*)zf, rc, out_split, (const DevState*)S->st);
       };
@@ -1792,13 +1777,13 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
     } else {
       const unsigned rb = blocks_for(sc.size(), 256, cap);
       if (bf(l) && bf(l + 1))
-        launch_pdl(k_restrict<T, D, BF, BF>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], (BF*)S->r[l + 1], S->st);
+        launch_pdl(k_restrict<T, BF, BF>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], (BF*)S->r[l + 1], S->st);
       else if (bf(l))
-        launch_pdl(k_restrict<T, D, BF, T>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], r[l + 1], S->st);
+        launch_pdl(k_restrict<T, BF, T>, rb, 256, 0, s, sh, sc, (const BF*)S->r[l], (const BF*)S->z[l], r[l + 1], S->st);
       else if (bf(l + 1))
-        launch_pdl(k_restrict<T, D, T, BF>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], (BF*)S->r[l + 1], S->st);
+        launch_pdl(k_restrict<T, T, BF>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], (BF*)S->r[l + 1], S->st);
       else
-        launch_pdl(k_restrict<T, D>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], r[l + 1], S->st);
+        launch_pdl(k_restrict<T>, rb, 256, 0, s, sh, sc, (const T*)r[l], (const T*)z[l], r[l + 1], S->st);
     }
   }
   const Shape sb = S->lv[L - 1];
@@ -1812,7 +1797,7 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
     const unsigned nb = blocks_for(sb.size(), 256, cap);
     int first = 1;
     auto pair = [&](int a, int b) {
-      if (first && a == 0) launch_pdl(k_smooth_first<T, D>, nb, 256, 0, s, sb, r[L - 1], z[L - 1], S->st, L == 1 ? 1 : 0);
+      if (first && a == 0) launch_pdl(k_smooth_first<T, D>, nb, 256, 0, s, sb, r[L - 1], z[L - 1], S->st, 0);
       else {
         if (first) cudaMemsetAsync(z[L - 1], 0, sizeof(T) * sb.size(), s);
         launch_pdl(k_smooth<T, D, false>, nb, 256, 0, s, sb, r[L - 1], z[L - 1], a, nullptr, S->st);
@@ -1835,8 +1820,7 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
       auto go = [&](auto* zf, auto* zc) {
         using SF = std::remove_pointer_t<decltype(zf)>;
         using SC = std::remove_pointer_t<decltype(zc)>;
-        const bool vec = two_aligned(zf, sizeof(SF), sh);
-        auto k = vec ? k_prolong_walk<T, SF, SC, kVec> : k_prolong_walk<T, SF, SC, kOne>;
+        auto k = k_prolong_walk<T, SF, SC, kVec>;
         if constexpr (kCanSplit) k = split ? k_prolong_walk<T, SF, SC, kSplit> : k;
         launch_pdl(k, (unsigned)w.items, kWalkBlock, 0, s, sh, sc, w, zf, (const SC*)zc, (int)(split && l + 1 < lc),
                    (const DevState*)S->st);
@@ -1848,13 +1832,13 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
     } else {
       const unsigned nb = blocks_for(sh.size(), 256, cap);
       if (bf(l) && bf(l + 1))
-        launch_pdl(k_prolong<T, D, BF, BF>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const BF*)S->z[l + 1], S->st);
+        launch_pdl(k_prolong<T, BF, BF>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const BF*)S->z[l + 1], S->st);
       else if (bf(l))
-        launch_pdl(k_prolong<T, D, BF, T>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const T*)z[l + 1], S->st);
+        launch_pdl(k_prolong<T, BF, T>, nb, 256, 0, s, sh, sc, (BF*)S->z[l], (const T*)z[l + 1], S->st);
       else if (bf(l + 1))
-        launch_pdl(k_prolong<T, D, T, BF>, nb, 256, 0, s, sh, sc, z[l], (const BF*)S->z[l + 1], S->st);
+        launch_pdl(k_prolong<T, T, BF>, nb, 256, 0, s, sh, sc, z[l], (const BF*)S->z[l + 1], S->st);
       else
-        launch_pdl(k_prolong<T, D>, nb, 256, 0, s, sh, sc, z[l], (const T*)z[l + 1], S->st);
+        launch_pdl(k_prolong<T>, nb, 256, 0, s, sh, sc, z[l], (const T*)z[l + 1], S->st);
     }
     for (int it = 0; it < P.pre_post; ++it) {
       sweep(l, 1);
@@ -1878,10 +1862,6 @@ static void launch_vcycle(fm_mgpcg* S, cudaStream_t s, bool dot_last, bool recen
       }
     }
   }
-  if (dot_last && L == 1) {
-    // single-level: z.r over the bottom result
-    launch_pdl(k_smooth<T, D, true>, kRedBlocks, kRedThreads, 0, s, sb, r[0], z[0], 2 /* no update */, S->part, S->st);
-  }
 }
 
 // x += alpha p, r -= alpha A p and the convergence test: the second half of a
@@ -1892,9 +1872,8 @@ static void launch_step(fm_mgpcg* S, cudaStream_t s) {
   const long n = s0.size();
   if constexpr (kWalkDots<T, D>) {
     const Walk w = walk_pairs(s0, kRedBlocks);
-    const bool vec = two_aligned(S->p, sizeof(T), s0) && two_aligned(S->Ap, sizeof(T), s0);
-    launch_pdl(vec ? k_Ap_walk<T, kVec> : k_Ap_walk<T, kOne>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock,
-               0, s, s0, w, (const T*)S->p, (T*)S->Ap, S->part, S->st);
+    launch_pdl(k_Ap_walk<T>, (unsigned)(w.items < kRedBlocks ? w.items : kRedBlocks), kWalkBlock, 0, s, s0, w, (const T*)S->p,
+               (T*)S->Ap, S->part, S->st);
   } else {
     launch_pdl(k_Ap_dot<T, D>, kRedBlocks, kRedThreads, 0, s, s0, (T*)S->p, (T*)S->Ap, S->part, S->st);
   }
