@@ -115,10 +115,10 @@ struct MarchJobs {
 };
 
 // One RK stage: velocity k = u(pos) and, with the Jacobian, d = (grad u)(pos) . t.
-template <typename T, int D, bool WT>
+template <typename T, int D, int RK, bool WT>
 __device__ __forceinline__ void march_eval(const Mac<T>& u, const fm_grid& g, const Q2Lim<T>& lim, const T* pos,
                                            const T* t, T inv_dx, T* k, T* d) {
-  if constexpr (WT) q2_mac_grad_dot<T, D>(u, g, lim, pos, inv_dx, t, k, d);
+  if constexpr (WT) q2_mac_grad_dot<T, D, RK == 4 && kNearest<T, true>>(u, g, lim, pos, inv_dx, t, k, d);
   else q2_mac_val<T, D>(u, g, lim, pos, inv_dx, k);
 }
 
@@ -139,11 +139,11 @@ __device__ __forceinline__ void march_node(const Mac<T>& u, const fm_grid& g, T 
   const T inv_dx = (T)1 / dx;
   const Q2Lim<T> lim(g);
   T k[3], d[3] = {0, 0, 0}, pos[3] = {0, 0, 0}, tt[3] = {0, 0, 0};
-  march_eval<T, D, WT>(u, g, lim, P, Tv, inv_dx, k, d);
+  march_eval<T, D, RK, WT>(u, g, lim, P, Tv, inv_dx, k, d);
   if constexpr (RK == 2) {
 #pragma unroll
     for (int a = 0; a < D; ++a) { pos[a] = P[a] + h * k[a]; tt[a] = Tv[a] + h * d[a]; }
-    march_eval<T, D, WT>(u, g, lim, pos, tt, inv_dx, k, d);
+    march_eval<T, D, RK, WT>(u, g, lim, pos, tt, inv_dx, k, d);
 #pragma unroll
     for (int a = 0; a < D; ++a) {
       psi[a * N + q] = P[a] + neg_dt * k[a];
@@ -158,7 +158,7 @@ __device__ __forceinline__ void march_node(const Mac<T>& u, const fm_grid& g, T 
       pos[a] = P[a] + h * k[a];
       tt[a] = Tv[a] + h * d[a];
     }
-    march_eval<T, D, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 2
+    march_eval<T, D, RK, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 2
 #pragma unroll
     for (int a = 0; a < D; ++a) {
       ks[a] = ks[a] + (T)2 * k[a];
@@ -166,7 +166,7 @@ __device__ __forceinline__ void march_node(const Mac<T>& u, const fm_grid& g, T 
       pos[a] = P[a] + h * k[a];
       tt[a] = Tv[a] + h * d[a];
     }
-    march_eval<T, D, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 3
+    march_eval<T, D, RK, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 3
 #pragma unroll
     for (int a = 0; a < D; ++a) {
       ks[a] = ks[a] + (T)2 * k[a];
@@ -174,7 +174,7 @@ __device__ __forceinline__ void march_node(const Mac<T>& u, const fm_grid& g, T 
       pos[a] = P[a] + (T)1.0 * neg_dt * k[a];
       tt[a] = Tv[a] + (T)1.0 * neg_dt * d[a];
     }
-    march_eval<T, D, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 4
+    march_eval<T, D, RK, WT>(u, g, lim, pos, tt, inv_dx, k, d);  // stage 4
     const T c6 = neg_dt * (T)1 / (T)6;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
