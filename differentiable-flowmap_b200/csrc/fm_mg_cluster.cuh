@@ -61,6 +61,8 @@ constexpr size_t kClMaxSmem = 226 * 1024;  // dynamic shared memory per CTA
 constexpr long kClDeepCells = 4096;        // CTA 0 alone smooths the levels of at most this many cells
 // Cells a CTA should hold before another CTA pays (whole solves, us for 1 / 2 / 4 / 8 / 16 CTAs: 64^2 151 135 133
 // 133 133, 128^2 354 . 266 232 230, 192^2 . . . 480 413, 32^3 . . . 205 184; a sequence of launches: 237, 361, 581, 221).
+// Up to where a solve fits the launches are slower: projections, launches / one cluster, 304^2 776 / 612, 368^2 821 /
+// 690, 512x272 822 / 764; FP64 176^2 353 / 263, 240^2 847 / 684; see plan_pcg_t for slabs that differ much.
 constexpr long kClCellsPerCta = 2048;
 
 // n / d for 0 <= n, d < 2^16 by one multiply: m = ceil(2^32 / d), 0 for d = 1.
@@ -1077,8 +1079,10 @@ inline bool cl_enable(Kernel kernel, int nc, size_t smem) {
   return cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
 }
 
-// Plans a whole solve in one cluster: returns the CTAs, or 0 where it does not
-// fit (the solve then runs as a sequence of launches).
+// Plans a whole solve in one cluster: returns the CTAs, or 0 (the solve then runs as a
+// sequence of launches) where the state does not fit 16 CTAs or level ld has fewer planes
+// than the CTAs that the cell count asks for.  With four levels and more that leaves squares
+// up to 384^2 (FP64: 240^2, masked 232^2) and cubes of 16^3, 24^3 and 32^3 (FP64: 16^3 and 24^3).
 template <typename Kernel>
 inline int cl_plan_pcg(ClArgs& a, Kernel kernel, const Shape* lv, int L, const fm_mg_params& P, int dim, size_t es,
                        bool solid, size_t* smem_out) {
