@@ -1675,12 +1675,12 @@ template <typename T, int D>
 static void plan_pcg_t(fm_mgpcg* S) {
   S->pcg_nc = cl_plan_pcg(S->pcg, k_pcg_cluster<T, D, false, DevState*>, S->lv, S->L, S->P, D, sizeof(T), false,
                           &S->pcg_smem);
-  // Near the top of the range the largest slab decides: with slabs that differ much the launches are as fast, where
-  // they have a coarse-level kernel (projections of five levels, us, launches / one cluster: 288x448 798 / 807, 320x448
-  // 768 / 781, 160x640 776 / 785; even slabs, 256x576 905 / 859, 480x320 916 / 891; without a coarse kernel, 336x448 on
-  // four levels, 2283 / 1845; slabs of less, 304x384 816 / 726).
+  // Near the top of the range the largest slab decides: where it is a fifth above the mean and over 10 500 cells the
+  // launches are as fast, if they have a coarse-level kernel (projections of five levels, us, launches / one cluster:
+  // 288x448 798 / 807, 320x448 768 / 781; smaller slabs, 400x320 868 / 821, 272x432 815 / 799, 304x384 816 / 726;
+  // without a coarse-level kernel, 400x352 on four levels, 2039 / 1618).
   const long slab = S->pcg_nc ? (long)S->pcg.lv[0].pmax * S->lv[0].s1 : 0;
-  if (D == 2 && sizeof(T) == 4 && S->lc > 0 && slab > 10000 && 5 * slab * S->pcg_nc >= 6 * S->lv[0].size()) S->pcg_nc = 0;
+  if (D == 2 && sizeof(T) == 4 && S->lc > 0 && slab > 10500 && 5 * slab * S->pcg_nc >= 6 * S->lv[0].size()) S->pcg_nc = 0;
 }
 
 static inline unsigned blocks_for(long n, int threads, long cap) {

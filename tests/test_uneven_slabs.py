@@ -1,4 +1,4 @@
-"""Whole solves of 2D FP32 grids whose largest slab holds over 10 000 cells, a fifth more
+"""Whole solves of 2D FP32 grids whose largest slab holds over 10 500 cells, a fifth more
 than the mean, run as a sequence of launches; even slabs, smaller ones and grids whose
 launches have no coarse-level kernel stay in one cluster."""
 import ctypes as C
@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape,levels,cluster", [
-    ((320, 448), 5, False), ((288, 448), 5, False), ((160, 640), 5, False),
-    ((480, 320), 5, True), ((304, 384), 5, True), ((336, 448), 4, True), ((384, 384), 5, True)])
+    ((320, 448), 5, False), ((288, 448), 5, False), ((400, 320), 5, True),
+    ((480, 320), 5, True), ((304, 384), 5, True), ((400, 352), 4, True), ((384, 384), 5, True)])
 def test_path(fm, cuda, shape, levels, cluster):
     lib, h, it = fm._lib.lib(), C.c_void_p(), C.c_int(0)
     P = fm._lib.MGParams(levels, 2, 10, 1, 200, 0.0, 1e-8, 1e-12, 4, 0)
