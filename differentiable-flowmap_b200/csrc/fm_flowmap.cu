@@ -118,7 +118,7 @@ struct MarchJobs {
 template <typename T, int D, int RK, bool WT>
 __device__ __forceinline__ void march_eval(const Mac<T>& u, const fm_grid& g, const Q2Lim<T>& lim, const T* pos,
                                            const T* t, T inv_dx, T* k, T* d) {
-  if constexpr (WT) q2_mac_grad_dot<T, D, RK == 4 && kNearest<T, true>>(u, g, lim, pos, inv_dx, t, k, d);
+  if constexpr (WT) q2_mac_grad_dot<T, D, RK == 4 && std::is_same<T, float>::value>(u, g, lim, pos, inv_dx, t, k, d);
   else q2_mac_val<T, D>(u, g, lim, pos, inv_dx, k);
 }
 

@@ -63,27 +63,29 @@ __device__ __forceinline__ double floor_pos(double s, int& i) {
 // 2^22: floor(s + 1/2), the floor taken by an addition of 2^23 rounded down (the
 // integer is in its mantissa) instead of a floor and a conversion, which run on
 // the quarter-rate XU pipe.  Exact: s + 1/2 rounds only where that cannot move
-// it across an integer.  Which kernels take it: kNearest.
+// it across an integer.
 __device__ __forceinline__ float nearest_pos(float s, int& i) {
   const float m = __fadd_rd(__fadd_rn(s, 0.5f), 8388608.0f);
   i = __float_as_int(m) - 0x4B000000;
   return __fadd_rn(m, -8388608.0f);
 }
+__device__ __forceinline__ double nearest_pos(double s, int& i) {
+  const double iu = floor(s), n = s - iu >= 0.5 ? iu + 1.0 : iu;
+  i = (int)n;
+  return n;
+}
 
-// FP32 kernels that take derivatives: the transposes (333 -> 310 us at 64^3) and the RK4 march
-// (three launches at 128^3: 2185 -> 2171 us).  The floor stays in the RK2 march (three launches at 128^3: 1242 us with it,
-// 1255 with the nearest node), in the kernels that read values only, which are bound by their L1
-// reads (0-1 % slower), and in FP64, where both take the same conversions (512^2 RK4 march 117
-// and 122 us, 90x77x101 RK2 772 and 777).
-template <typename T, bool GRAD>
-constexpr bool kNearest = GRAD && std::is_same<T, float>::value;
-
+// NEAR: the kernels that take it are those with derivatives, namely the transposes (advection adjoints at
+// 64^3, RK4, FP32 333 -> 310 us, FP64 511 -> 394) and the FP32 RK4 march (three launches at 128^3: 2185 ->
+// 2171).  The floor stays in the kernels that read values only, which are bound by their L1 reads (0-1 %
+// slower with the nearest node), in the RK2 march (128^3, FP32: 1242 with the floor, 1255 with the nearest
+// node) and in the FP64 march (512^2 RK4 117 and 122, 90x77x101 RK2 772 and 777).
 template <typename T, bool GRAD>
 struct Q2 {
   int i0;
   T w0, w1, w2;
   T d0, d1, d2;
-  template <bool NEAR = kNearest<T, GRAD>>
+  template <bool NEAR = GRAD>
   __device__ __forceinline__ void setup(T pos_scaled, T bl, T hi) {
     const T u = pos_scaled - bl;
     T s = u < hi ? u : hi;
@@ -267,7 +269,7 @@ template <typename T, int D, bool G>
 struct MacStencil {
   Q2<T, G> s0[3];  // BL = 0
   Q2<T, G> s5[3];  // BL = 0.5
-  template <bool NEAR = kNearest<T, G>>
+  template <bool NEAR = G>
   __device__ __forceinline__ void setup(const Q2Lim<T>& lim, const T* p, T inv_dx) {
 #pragma unroll
     for (int a = 0; a < D; ++a) {
@@ -302,7 +304,7 @@ struct CompStencil {
 };
 
 // value v = u(p) and d = (grad u)(p) . t (RK_grid's Jacobian update)
-template <typename T, int D, bool NEAR = kNearest<T, true>>
+template <typename T, int D, bool NEAR = true>
 __device__ __forceinline__ void q2_mac_grad_dot(const Mac<T>& u, const fm_grid& g, const Q2Lim<T>& lim, const T* p,
                                                 T inv_dx, const T* t, T* v, T* d) {
   MacStencil<T, D, true> st;
