@@ -59,35 +59,44 @@ struct PointAdj {
 // two more at the chain's end instead of three per lane (the L2's atomic
 // throughput bounds these kernels; RK4 advection adjoint at 64^3, FP32: 308 -> 241 us).  key: a lane's
 // first flat index; a lane that scatters nothing (live = false) takes part in the
-// shuffles only.  Every lane of the warp calls these.
+// shuffles only.  Every lane of the warp calls these.  !ON: three atomics per lane, by any
+// lanes.
+template <bool ON>
 struct Chain {
   bool live, linked, last;  // linked: the lane before continues into this one
-  __device__ __forceinline__ Chain(unsigned key, bool lv) : live(lv) {
-    constexpr unsigned all = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const unsigned before = __shfl_up_sync(all, key, 1);
-    const unsigned lives = __ballot_sync(all, live);
-    linked = live && lane > 0 && ((lives >> (lane - 1)) & 1) && before + 1 == key;
-    const unsigned links = __ballot_sync(all, linked);
-    last = live && !(lane < 31 && ((links >> (lane + 1)) & 1));
+  __device__ __forceinline__ Chain(unsigned key, bool lv) : live(lv), linked(false), last(lv) {
+    if constexpr (ON) {
+      constexpr unsigned all = 0xffffffffu;
+      const int lane = threadIdx.x & 31;
+      const unsigned before = __shfl_up_sync(all, key, 1);
+      const unsigned lives = __ballot_sync(all, live);
+      linked = live && lane > 0 && ((lives >> (lane - 1)) & 1) && before + 1 == key;
+      const unsigned links = __ballot_sync(all, linked);
+      last = live && !(lane < 31 && ((links >> (lane + 1)) & 1));
+    }
   }
   // p[0..2] += a0, a1, a2
   template <typename T>
   __device__ __forceinline__ void add(T* p, T a0, T a1, T a2) const {
-    constexpr unsigned all = 0xffffffffu;
-    const T b2 = __shfl_up_sync(all, a2, 1);
-    const T m = linked ? a1 + b2 : a1;  // all this chain adds to p[1] up to this lane
-    const T bm = __shfl_up_sync(all, m, 1);
-    if (live) atomicAdd(p, linked ? a0 + bm : a0);
+    if constexpr (ON) {
+      constexpr unsigned all = 0xffffffffu;
+      const T b2 = __shfl_up_sync(all, a2, 1);
+      const T m = linked ? a1 + b2 : a1;  // all this chain adds to p[1] up to this lane
+      const T bm = __shfl_up_sync(all, m, 1);
+      if (live) atomicAdd(p, linked ? a0 + bm : a0);
+      a1 = m;
+    } else {
+      if (live) atomicAdd(p, a0);
+    }
     if (last) {
-      atomicAdd(p + 1, m);
+      atomicAdd(p + 1, a1);
       atomicAdd(p + 2, a2);
     }
   }
 };
 
 // f[taps] += val * w(p) where live; every lane of the warp calls it
-template <typename T, int D>
+template <typename T, int D, bool CHAIN>
 __device__ __forceinline__ void scatter(T* f, const Shape& s, const PointAdj<T, D>& P, T val, bool live) {
   const Q2<T, true>& x = P.ax[0].q;
   const Q2<T, true>& y = P.ax[1].q;
@@ -96,7 +105,7 @@ __device__ __forceinline__ void scatter(T* f, const Shape& s, const PointAdj<T, 
     const Q2<T, true>& z = P.ax[2].q;
     const unsigned sj = s.s2, si = (unsigned)s.s1 * s.s2;
     const unsigned b = ((unsigned)x.i0 * s.s1 + y.i0) * s.s2 + z.i0;
-    const Chain ch(b, live);
+    const Chain<CHAIN> ch(b, live);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const T vi = val * wx[i];
@@ -109,7 +118,7 @@ __device__ __forceinline__ void scatter(T* f, const Shape& s, const PointAdj<T, 
   } else {
     const unsigned si = s.s1;
     const unsigned b = (unsigned)x.i0 * s.s1 + y.i0;
-    const Chain ch(b, live);
+    const Chain<CHAIN> ch(b, live);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const T vi = val * wx[i];
@@ -130,7 +139,8 @@ __device__ __forceinline__ void val_grad(const T* __restrict__ f, const Shape& s
 
 // One RK stage of a backtrace in reverse: the stage sampled u0 at q, its
 // adjoint vbar scatters into gu0 (when wanted) and qbar = (d u0(q) / d q)^T vbar.
-template <typename T, int D>
+// SKIP: lanes that are not live take no samples.
+template <typename T, int D, bool SKIP>
 __device__ __forceinline__ void stage_adj(const Mac<T>& u0, const MacW<T>& gu0, const fm_grid& g,
                                           const Q2Lim<T>& lim, const T* q, T inv_dx, const T* vbar, bool want_q,
                                           T* qbar, bool live) {
@@ -141,8 +151,8 @@ __device__ __forceinline__ void stage_adj(const Mac<T>& u0, const MacW<T>& gu0, 
     PointAdj<T, D> P;
     P.setup(lim, c, q, inv_dx);
     const Shape s = face_shape(g, c);
-    scatter<T, D>(gu0.c[c], s, P, vbar[c], live);
-    if (want_q) {
+    scatter<T, D, true>(gu0.c[c], s, P, vbar[c], live);
+    if (want_q && (!SKIP || live)) {
       T v, gp[3];
       val_grad<T, D>(u0.c[c], s, P, inv_dx, v, gp);
 #pragma unroll
@@ -187,7 +197,7 @@ __device__ __forceinline__ void backtrace_stages(const Mac<T>& u0, const fm_grid
 //   RK2: p = X - dt v2, q1 = X - dt/2 v1
 //   RK4: p = X - dt/6 (v1 + 2 v2 + 2 v3 + v4), q1 = X - dt/2 v1, q2 = X - dt/2 v2,
 //        q3 = X - dt v3
-template <typename T, int D, int RK>
+template <typename T, int D, int RK, bool SKIP>
 __device__ __forceinline__ void backtrace_adj(const Mac<T>& u0, const MacW<T>& gu0, const fm_grid& g,
                                               const Q2Lim<T>& lim, T q[4][3], T inv_dx, T dt, const T* pbar,
                                               bool live) {
@@ -195,24 +205,24 @@ __device__ __forceinline__ void backtrace_adj(const Mac<T>& u0, const MacW<T>& g
   if constexpr (RK == 2) {
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = -dt * pbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[1], inv_dx, vbar, true, qbar, live);
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[1], inv_dx, vbar, true, qbar, live);
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = (T)-0.5 * dt * qbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[0], inv_dx, vbar, false, qbar, live);
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[0], inv_dx, vbar, false, qbar, live);
   } else {
     const T w16 = -dt / (T)6, w13 = -dt / (T)3;
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = w16 * pbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[3], inv_dx, vbar, true, qbar, live);  // v4 at q3
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[3], inv_dx, vbar, true, qbar, live);  // v4 at q3
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = w13 * pbar[a] - dt * qbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[2], inv_dx, vbar, true, qbar, live);  // v3 at q2
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[2], inv_dx, vbar, true, qbar, live);  // v3 at q2
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = w13 * pbar[a] + (T)-0.5 * dt * qbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[1], inv_dx, vbar, true, qbar, live);  // v2 at q1
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[1], inv_dx, vbar, true, qbar, live);  // v2 at q1
 #pragma unroll
     for (int a = 0; a < D; ++a) vbar[a] = w16 * pbar[a] + (T)-0.5 * dt * qbar[a];
-    stage_adj<T, D>(u0, gu0, g, lim, q[0], inv_dx, vbar, false, qbar, live);  // v1 at X
+    stage_adj<T, D, SKIP>(u0, gu0, g, lim, q[0], inv_dx, vbar, false, qbar, live);  // v1 at X
   }
 }
 
@@ -230,26 +240,72 @@ __global__ void __launch_bounds__(kAdjThreads) k_advect_grid_adj(fm_grid g, T dx
   const long n0 = (long)blockIdx.x * blockDim.x + threadIdx.x, n = n0 < s.size() ? n0 : s.size() - 1;
   const T lam = pick(gout, slot)[n];
   // a zero adjoint contributes nothing to either gradient; its lane only keeps
-  // the warp whole for the scatters
+  // the warp whole for the scatters.  Whether it samples: in FP64 RK2 it does not (velocity at 64^3, us, dense
+  // and with 1 % of the adjoint not zero, without / with its samples: 183, 90 / 197, 106; RK4 402, 225 / 392,
+  // 219; FP32 the same within 1 %).  A second body for warps of few lanes, lane by lane, made the dense ones
+  // slower (FP64 164 -> 212 us at 40x61x90, RK2: instruction fetch).
   const bool live = n0 < s.size() && lam != (T)0;
   if (!__any_sync(0xffffffffu, live)) return;
+  constexpr bool kSkip = sizeof(T) == 8 && RK == 2;
+  const bool samples = !kSkip || live;
   int i, j, k;
   unflatten(s, n, i, j, k);
-  T X[3] = {0, 0, 0}, p[3] = {0, 0, 0}, q[4][3];
+  T X[3] = {0, 0, 0}, p[3] = {0, 0, 0}, q[4][3] = {};
   node_pos<T, D>(c, i, j, k, dx, X);
   const T inv_dx = (T)1 / dx;
   const Q2Lim<T> lim(g);
-  backtrace_stages<T, D, RK>(u0, g, lim, X, inv_dx, dt, q, p);
+  if (samples) backtrace_stages<T, D, RK>(u0, g, lim, X, inv_dx, dt, q, p);
   PointAdj<T, D> P;
   P.setup(lim, c, p, inv_dx);
   T* gf = pick(gf1, slot);
-  if (gf != nullptr) scatter<T, D>(gf, s, P, lam, live);
+  if (gf != nullptr) scatter<T, D, true>(gf, s, P, lam, live);
   if (gu0.c[0] == nullptr) return;
   T v, gp[3] = {0, 0, 0}, pbar[3] = {0, 0, 0};
-  val_grad<T, D>(pick(f1, slot), s, P, inv_dx, v, gp);
+  if (samples) val_grad<T, D>(pick(f1, slot), s, P, inv_dx, v, gp);
 #pragma unroll
   for (int a = 0; a < D; ++a) pbar[a] = lam * gp[a];
-  backtrace_adj<T, D, RK>(u0, gu0, g, lim, q, inv_dx, dt, pbar, live);
+  backtrace_adj<T, D, RK, kSkip>(u0, gu0, g, lim, q, inv_dx, dt, pbar, live);
+}
+
+// How the warps of the pullbacks go by their adjoint: one without any is done, one with few
+// neighbouring lanes that have one lets the others go and scatters lane by lane, the others
+// chain (velocity at 40x61x90, FP32, us, chained only / so: 1 % of the adjoint not zero
+// 28.7 / 19.8, a quarter 74 / 64, dense 124 / 119).
+enum { kNone, kPlain, kChained };
+__device__ __forceinline__ int scatter_form(bool live) {
+  const unsigned lives = __ballot_sync(0xffffffffu, live);
+  return lives == 0 ? kNone : (__popc(lives & (lives << 1)) < 8 ? kPlain : kChained);
+}
+
+template <typename T, int D, bool CHAIN>
+__device__ __forceinline__ void pullback_u_adj_node(const fm_grid& g, T dx, long N, long n, T al, bool live,
+                                                    const Mac<T>& u0, const T* T_c, const T* psi_c, const MacW<T>& gu0,
+                                                    T* gT_c, T* gp_c) {
+  T p[3] = {0, 0, 0}, t[3] = {0, 0, 0};
+#pragma unroll
+  for (int a = 0; a < D; ++a) p[a] = psi_c[a * N + n], t[a] = T_c[a * N + n];
+  const T inv_dx = (T)1 / dx;
+  const Q2Lim<T> lim(g);
+  T pbar[3] = {0, 0, 0};
+  const bool want_v = gT_c != nullptr || gp_c != nullptr;
+#pragma unroll
+  for (int a = 0; a < D; ++a) {
+    PointAdj<T, D> P;
+    P.setup(lim, a, p, inv_dx);
+    const Shape sa = face_shape(g, a);
+    if (gu0.c[0] != nullptr) scatter<T, D, CHAIN>(gu0.c[a], sa, P, al * t[a], live);
+    if (want_v) {
+      T v, gp[3] = {0, 0, 0};
+      val_grad<T, D>(u0.c[a], sa, P, inv_dx, v, gp);
+      if (gT_c != nullptr && live) gT_c[a * N + n] += al * v;
+#pragma unroll
+      for (int b = 0; b < D; ++b) pbar[b] += al * t[a] * gp[b];
+    }
+  }
+  if (gp_c != nullptr && live) {
+#pragma unroll
+    for (int b = 0; b < D; ++b) gp_c[b * N + n] += pbar[b];
+  }
 }
 
 // Adjoint of out_c = alpha (T_c . u0(psi_c) + beta base_c) on face grid
@@ -259,40 +315,37 @@ __global__ void __launch_bounds__(kAdjThreads) k_pullback_u_adj(fm_grid g, T dx,
                                                                 T alpha, T beta, Mac<T> gout, MacW<T> gu0,
                                                                 MacW<T> gT, MacW<T> gpsi, MacW<T> gbase) {
   const int c = blockIdx.y;
-  const Shape s = face_shape(g, c);
-  const long N = s.size();
+  const long N = face_shape(g, c).size();
   const long n0 = (long)blockIdx.x * blockDim.x + threadIdx.x, n = n0 < N ? n0 : N - 1;
   const T al = alpha * pick(gout, c)[n];
   if (gbase.c[0] != nullptr && n0 < N) pick(gbase, c)[n] += al * beta;
   const bool live = n0 < N && al != (T)0;
-  if (!__any_sync(0xffffffffu, live)) return;
-  const T* psi_c = pick(psi, c);
-  const T* T_c = pick(Tm, c);
-  T p[3] = {0, 0, 0}, t[3] = {0, 0, 0};
+  const int form = scatter_form(live);
+  const T* const T_c = pick(Tm, c);
+  const T* const psi_c = pick(psi, c);
+  T* const gT_c = gT.c[0] != nullptr ? pick(gT, c) : nullptr;
+  T* const gp_c = gpsi.c[0] != nullptr ? pick(gpsi, c) : nullptr;
+  if (form == kChained) pullback_u_adj_node<T, D, true>(g, dx, N, n, al, live, u0, T_c, psi_c, gu0, gT_c, gp_c);
+  else if (live) pullback_u_adj_node<T, D, false>(g, dx, N, n, al, true, u0, T_c, psi_c, gu0, gT_c, gp_c);
+}
+
+template <typename T, int D, bool CHAIN>
+__device__ __forceinline__ void pullback_scalar_adj_node(const fm_grid& g, T dx, const Shape& s, long n, T al, bool live,
+                                                         const T* s0, const T* psi, T* gs0, T* gpsi) {
+  const long N = s.size();
+  T p[3] = {0, 0, 0};
 #pragma unroll
-  for (int a = 0; a < D; ++a) p[a] = psi_c[a * N + n], t[a] = T_c[a * N + n];
+  for (int a = 0; a < D; ++a) p[a] = psi[a * N + n];
   const T inv_dx = (T)1 / dx;
   const Q2Lim<T> lim(g);
-  T pbar[3] = {0, 0, 0};
-  const bool want_v = gT.c[0] != nullptr || gpsi.c[0] != nullptr;
+  PointAdj<T, D> P;
+  P.setup(lim, -1, p, inv_dx);
+  if (gs0 != nullptr) scatter<T, D, CHAIN>(gs0, s, P, al, live);
+  if (gpsi != nullptr && live) {
+    T v, gp[3] = {0, 0, 0};
+    val_grad<T, D>(s0, s, P, inv_dx, v, gp);
 #pragma unroll
-  for (int a = 0; a < D; ++a) {
-    PointAdj<T, D> P;
-    P.setup(lim, a, p, inv_dx);
-    const Shape sa = face_shape(g, a);
-    if (gu0.c[0] != nullptr) scatter<T, D>(gu0.c[a], sa, P, al * t[a], live);
-    if (want_v) {
-      T v, gp[3] = {0, 0, 0};
-      val_grad<T, D>(u0.c[a], sa, P, inv_dx, v, gp);
-      if (gT.c[0] != nullptr && live) pick(gT, c)[a * N + n] += al * v;
-#pragma unroll
-      for (int b = 0; b < D; ++b) pbar[b] += al * t[a] * gp[b];
-    }
-  }
-  if (gpsi.c[0] != nullptr && live) {
-    T* gp_c = pick(gpsi, c);
-#pragma unroll
-    for (int b = 0; b < D; ++b) gp_c[b * N + n] += pbar[b];
+    for (int b = 0; b < D; ++b) gpsi[b * N + n] += al * gp[b];
   }
 }
 
@@ -308,21 +361,9 @@ __global__ void __launch_bounds__(kAdjThreads) k_pullback_scalar_adj(fm_grid g, 
   const T al = alpha * gout[n];
   if (gbase != nullptr && n0 < N) gbase[n] += al * beta;
   const bool live = n0 < N && al != (T)0;
-  if (!__any_sync(0xffffffffu, live)) return;
-  T p[3] = {0, 0, 0};
-#pragma unroll
-  for (int a = 0; a < D; ++a) p[a] = psi[a * N + n];
-  const T inv_dx = (T)1 / dx;
-  const Q2Lim<T> lim(g);
-  PointAdj<T, D> P;
-  P.setup(lim, -1, p, inv_dx);
-  if (gs0 != nullptr) scatter<T, D>(gs0, s, P, al, live);
-  if (gpsi != nullptr && live) {
-    T v, gp[3] = {0, 0, 0};
-    val_grad<T, D>(s0, s, P, inv_dx, v, gp);
-#pragma unroll
-    for (int b = 0; b < D; ++b) gpsi[b * N + n] += al * gp[b];
-  }
+  const int form = scatter_form(live);
+  if (form == kChained) pullback_scalar_adj_node<T, D, true>(g, dx, s, n, al, live, s0, psi, gs0, gpsi);
+  else if (live) pullback_scalar_adj_node<T, D, false>(g, dx, s, n, al, true, s0, psi, gs0, gpsi);
 }
 
 // ---------------------------------------------------------------------------
@@ -400,7 +441,7 @@ __device__ __forceinline__ void val_grad_hess(const T* __restrict__ f, const Sha
 
 // f[taps] += kv * w + kd * (grad w . t)   (value and directional-derivative
 // adjoints; the derivative weights unmasked, as the forward's d uses them)
-template <typename T, int D>
+template <typename T, int D, bool CHAIN>
 __device__ __forceinline__ void scatter_vd(T* f, const Shape& s, const PointAdj<T, D>& P, T inv_dx, T kv, T kd,
                                            const T* t, bool live) {
   T w[3][3], e[3][3];  // e = derivative weight * t_a / dx
@@ -414,7 +455,7 @@ __device__ __forceinline__ void scatter_vd(T* f, const Shape& s, const PointAdj<
   if constexpr (D == 3) {
     const unsigned sj = s.s2, si = (unsigned)s.s1 * s.s2;
     const unsigned b = ((unsigned)P.ax[0].q.i0 * s.s1 + P.ax[1].q.i0) * s.s2 + P.ax[2].q.i0;
-    const Chain ch(b, live);
+    const Chain<CHAIN> ch(b, live);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -431,7 +472,7 @@ __device__ __forceinline__ void scatter_vd(T* f, const Shape& s, const PointAdj<
   } else {
     const unsigned si = s.s1;
     const unsigned b = (unsigned)P.ax[0].q.i0 * s.s1 + P.ax[1].q.i0;
-    const Chain ch(b, live);
+    const Chain<CHAIN> ch(b, live);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       T r[3];
@@ -448,7 +489,7 @@ __device__ __forceinline__ void scatter_vd(T* f, const Shape& s, const PointAdj<
 
 // One march stage in reverse: k = u(pos), d = (grad u)(pos) t with adjoints
 // kbar, dbar (dbar unused when !WT) -> posbar, tbar; u's gradient scattered.
-template <typename T, int D, bool WT>
+template <typename T, int D, bool WT, bool CHAIN>
 __device__ __forceinline__ void march_stage_adj(const Mac<T>& u, const MacW<T>& gu, const fm_grid& g,
                                                 const Q2Lim<T>& lim, const T* pos, const T* t, T inv_dx,
                                                 const T* kbar, const T* dbar, T* posbar, T* tbar, bool live) {
@@ -467,12 +508,12 @@ __device__ __forceinline__ void march_stage_adj(const Mac<T>& u, const MacW<T>& 
         posbar[a] += kbar[c] * gr[a] + dbar[c] * Ht[a];
         tbar[a] += dbar[c] * graw[a];
       }
-      if (gu.c[0] != nullptr) scatter_vd<T, D>(gu.c[c], s, P, inv_dx, kbar[c], dbar[c], t, live);
+      if (gu.c[0] != nullptr) scatter_vd<T, D, CHAIN>(gu.c[c], s, P, inv_dx, kbar[c], dbar[c], t, live);
     } else {
       val_grad<T, D>(u.c[c], s, P, inv_dx, v, gr);
 #pragma unroll
       for (int a = 0; a < D; ++a) posbar[a] += kbar[c] * gr[a];
-      if (gu.c[0] != nullptr) scatter<T, D>(gu.c[c], s, P, kbar[c], live);
+      if (gu.c[0] != nullptr) scatter<T, D, CHAIN>(gu.c[c], s, P, kbar[c], live);
     }
   }
 }
@@ -494,6 +535,9 @@ __global__ void __launch_bounds__(kAdjThreads) k_march_adj(fm_grid g, T dx, T dt
   const long n0 = (long)blockIdx.x * blockDim.x + threadIdx.x, n = n0 < N ? n0 : N - 1;
   const bool live = n0 < N;  // a lane past the end only keeps its warp whole for the scatters
   constexpr int S = RK == 2 ? 2 : 4;
+  // RK4 in FP64 is bound by its arithmetic in 3D, not by the atomics (64^3 418 us chained, 386 lane by lane;
+  // 250x333 24.7 and 26.7)
+  constexpr bool kChain = !(D == 3 && RK == 4 && sizeof(T) == 8);
   T P0[3] = {0, 0, 0}, T0[3] = {0, 0, 0}, Pb[3] = {0, 0, 0}, Tb[3] = {0, 0, 0};
 #pragma unroll
   for (int a = 0; a < D; ++a) {
@@ -528,13 +572,13 @@ __global__ void __launch_bounds__(kAdjThreads) k_march_adj(fm_grid g, T dx, T dt
   if constexpr (RK == 2) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) kb[a] = neg_dt * Pb[a], db[a] = neg_dt * Tb[a];
-    march_stage_adj<T, D, WT>(u, gu, g, lim, pos[1], tt[1], inv_dx, kb, db, pb, tb, live);
+    march_stage_adj<T, D, WT, kChain>(u, gu, g, lim, pos[1], tt[1], inv_dx, kb, db, pb, tb, live);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       kb[a] = h * pb[a], db[a] = h * tb[a];
       Pb[a] += pb[a], Tb[a] += tb[a];
     }
-    march_stage_adj<T, D, WT>(u, gu, g, lim, pos[0], tt[0], inv_dx, kb, db, pb, tb, live);
+    march_stage_adj<T, D, WT, kChain>(u, gu, g, lim, pos[0], tt[0], inv_dx, kb, db, pb, tb, live);
   } else {
     const T c6 = neg_dt * (T)1 / (T)6;
     const T Po[3] = {Pb[0], Pb[1], Pb[2]}, To[3] = {Tb[0], Tb[1], Tb[2]};
@@ -542,7 +586,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_march_adj(fm_grid g, T dx, T dt
     for (int a = 0; a < 3; ++a) kb[a] = c6 * Po[a], db[a] = c6 * To[a];
 #pragma unroll
     for (int st = 3; st >= 1; --st) {
-      march_stage_adj<T, D, WT>(u, gu, g, lim, pos[st], tt[st], inv_dx, kb, db, pb, tb, live);
+      march_stage_adj<T, D, WT, kChain>(u, gu, g, lim, pos[st], tt[st], inv_dx, kb, db, pb, tb, live);
       const T hs = st == 3 ? neg_dt : h;        // how stage st's state depends on the previous stage's k, d
       const T wprev = st == 1 ? c6 : (T)2 * c6;  // weight of the previous stage's k, d in the update
 #pragma unroll
@@ -552,7 +596,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_march_adj(fm_grid g, T dx, T dt
         db[a] = wprev * To[a] + hs * tb[a];
       }
     }
-    march_stage_adj<T, D, WT>(u, gu, g, lim, pos[0], tt[0], inv_dx, kb, db, pb, tb, live);
+    march_stage_adj<T, D, WT, kChain>(u, gu, g, lim, pos[0], tt[0], inv_dx, kb, db, pb, tb, live);
   }
 #pragma unroll
   for (int a = 0; a < D; ++a) {
