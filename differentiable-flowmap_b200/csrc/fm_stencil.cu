@@ -97,6 +97,18 @@ __device__ __forceinline__ void copy_async(T* dst, const T* src) {
                : "memory");
 }
 
+// Shared memory of a 3D tile: footprints, the pairs after the k pass and those after the j
+// pass; the latter lie over the footprints where all three do not fit (kOwnB false: FP64
+// cubic and quartic tiles 8 high with margins), which then arrive after the i pass.
+template <typename T, int ORDER, int M, int TI>
+struct Fixed3 {
+  static constexpr int NZ = Taps<ORDER>::nz;
+  static constexpr int FI = TI + NZ - 1 + 2 * M, FJ = kTJ3 + NZ - 1 + 2 * M, FK = kTK3 + NZ - 1 + 2 * M;
+  static constexpr size_t front = sizeof(T) * (2 * FI * FJ * FK + 2 * FI * FJ * kTK3), b = sizeof(T) * 2 * FI * kTJ3 * kTK3;
+  static constexpr bool kOwnB = front + b <= 227 * 1024 - 8192;  // the tables are static
+  static constexpr size_t smem = front + (kOwnB ? b : 0);
+};
+
 // Per tile and term, the footprints of both fields are contracted along k (a warp
 // per row; a lane's k and so its weights stay in registers), then, as pairs, along
 // j and i with one column per thread held in registers: n outputs of a column cost
@@ -115,8 +127,9 @@ template <typename T, int ORDER, int M, int TI3>
 __global__ void __launch_bounds__(kStThreads, 2) k_fixed_grad_dot3(fm_grid g, T dx, StTerms<T> terms, MacW<T> outs) {
   constexpr int NZ = Taps<ORDER>::nz;
   constexpr int TI = TI3, TJ = kTJ3, TK = kTK3;
-  // footprint: taps from the tile's first base - M (see fixed3_smem)
-  constexpr int FI = TI + NZ - 1 + 2 * M, FJ = TJ + NZ - 1 + 2 * M, FK = TK + NZ - 1 + 2 * M;
+  // footprint: taps from the tile's first base - M (see launch_fixed3)
+  using L3 = Fixed3<T, ORDER, M, TI>;
+  constexpr int FI = L3::FI, FJ = L3::FJ, FK = L3::FK;
   constexpr int WARPS = kStThreads / 32;
   static_assert(TK == 32 && TJ == WARPS, "a warp is a row along k; an i column per thread");
   using W = TapWeights<T, NZ>;
@@ -125,7 +138,7 @@ __global__ void __launch_bounds__(kStThreads, 2) k_fixed_grad_dot3(fm_grid g, T 
   extern __shared__ __align__(16) unsigned char st_smem[];
   P* sA = reinterpret_cast<P*>(st_smem);
   P* sB = sA + FI * FJ * TK;
-  T* sF = reinterpret_cast<T*>(sB + FI * TJ * TK);
+  T* sF = reinterpret_cast<T*>(L3::kOwnB ? sB + FI * TJ * TK : sB);
   T* sH = sF + FI * FJ * FK;
   struct Tables {
     W wI[TI], wJ[TJ], wK[TK];
@@ -225,7 +238,7 @@ __global__ void __launch_bounds__(kStThreads, 2) k_fixed_grad_dot3(fm_grid g, T 
     }
     if (a + 1 < terms.n) tables(a + 1);
     __syncthreads();
-    if (a + 1 < terms.n) load(a + 1);
+    if (L3::kOwnB && a + 1 < terms.n) load(a + 1);
     // j pass
     for (int ii = warp; ii < FI; ii += WARPS) {
       const P* Ac = sA + ii * FJ * TK + lane;
@@ -279,6 +292,10 @@ __global__ void __launch_bounds__(kStThreads, 2) k_fixed_grad_dot3(fm_grid g, T 
         for (int q = 0; q < NZ; ++q) pair_fma(s, Bc[(off + q) * TJ * TK], w.v[q]);
         acc[i] += (s.f * inv_dx) * s.h;
       }
+    }
+    if (!L3::kOwnB && a + 1 < terms.n) {
+      __syncthreads();  // the i pass has read what the footprints overwrite
+      load(a + 1);
     }
   }
   const int k = k0 + lane, j = j0 + warp;
@@ -376,13 +393,6 @@ __global__ void __launch_bounds__(kStThreads) k_fixed_grad_dot2(fm_grid g, T dx,
 // lie within [b0, b0 + n - 1] of the first node's b0 (M = 0).  Otherwise the
 // quotient carries a rounding error and they lie within [b0 - 1, b0 + n]: the
 // footprints then hold n + NZ + 1 taps from b0 - 1 (M = 1).
-template <typename T, int ORDER, int M, int TI>
-static constexpr size_t fixed3_smem() {
-  constexpr int NZ = Taps<ORDER>::nz;
-  constexpr int FI = TI + NZ - 1 + 2 * M, FJ = kTJ3 + NZ - 1 + 2 * M, FK = kTK3 + NZ - 1 + 2 * M;
-  return sizeof(T) * (2 * FI * FJ * FK + 2 * FI * FJ * kTK3 + 2 * FI * kTJ3 * kTK3);
-}
-
 static bool power_of_two(double x) {
   int e;
   return x > 0 && std::frexp(x, &e) == 0.5;
@@ -390,7 +400,8 @@ static bool power_of_two(double x) {
 
 template <typename T, int ORDER, int M, int TI>
 static void launch_fixed3(const fm_grid& g, T dx, const StTerms<T>& terms, const MacW<T>& out, cudaStream_t s) {
-  const size_t smem = fixed3_smem<T, ORDER, M, TI>();
+  constexpr size_t smem = Fixed3<T, ORDER, M, TI>::smem;
+  static_assert(smem <= 227 * 1024 - 8192, "fits a CTA");
   if (!raise_smem_limit(k_fixed_grad_dot3<T, ORDER, M, TI>, smem)) return;
   dim3 grid(3 * ((g.n[2] + kTK3) / kTK3), (g.n[1] + kTJ3) / kTJ3, (g.n[0] + TI) / TI);  // face grids: up to n + 1
   launch(k_fixed_grad_dot3<T, ORDER, M, TI>, grid, kStThreads, smem, s, g, dx, terms, out);
@@ -404,12 +415,11 @@ static void launch_fixed(const fm_grid& g, T dx, const StTerms<T>& terms, const 
   const int ti = tuned_value(FM_TUNE_ADJ_SOURCE_TILE, g, g.dim == 3 ? 8 : 16);
   const bool exact = power_of_two((double)dx);
   if (g.dim == 3) {
-    // (with margins, FP64 cubic and quartic tiles 8 high would need over 227 KB of shared memory)
     if (exact) {
       if (ti == 4) launch_fixed3<T, ORDER, 0, 4>(g, dx, terms, out, s);
       else launch_fixed3<T, ORDER, 0, 8>(g, dx, terms, out, s);
     } else {
-      if (ti == 4 || fixed3_smem<T, ORDER, 1, 8>() > 227 * 1024) launch_fixed3<T, ORDER, 1, 4>(g, dx, terms, out, s);
+      if (ti == 4) launch_fixed3<T, ORDER, 1, 4>(g, dx, terms, out, s);
       else launch_fixed3<T, ORDER, 1, 8>(g, dx, terms, out, s);
     }
     return;
