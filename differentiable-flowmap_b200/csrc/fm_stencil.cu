@@ -99,7 +99,8 @@ __device__ __forceinline__ void copy_async(T* dst, const T* src) {
 
 // Shared memory of a 3D tile: footprints, the pairs after the k pass and those after the j
 // pass; the latter lie over the footprints where all three do not fit (kOwnB false: FP64
-// cubic and quartic tiles 8 high with margins), which then arrive after the i pass.
+// cubic and quartic tiles 8 high with margins), which then arrive after the i pass
+// (nabla_u_w at 40x61x90, order 3 / 4: 80 / 117 us; 111 / 177 by tiles 4 high).
 template <typename T, int ORDER, int M, int TI>
 struct Fixed3 {
   static constexpr int NZ = Taps<ORDER>::nz;
