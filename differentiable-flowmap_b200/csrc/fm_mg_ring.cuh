@@ -1,7 +1,7 @@
 // fm_mg_ring.cuh -- the coarse end of the MG V-cycle in one cluster launch, natural order.
 //
 // Included by fm_mgpcg.cu (needs DevState, kMaxLevels).  The job of k_mg_ring
-// (fm_mg_cluster.cuh) for 2D grids and in FP64, where its branch-free quotients and
+// (fm_mg_cluster.cuh) for most 2D grids and in FP64, where its branch-free quotients and
 // its push exchange do not pay (us a V-cycle, this / that one: FP64 40^3 69 / 72, 384^2
 // 77 / 83, 64^2 47 / 52; FP32 512^2 79.4 / 80.2; FP32 40^3 62 / 60, 128^3 142 / 126).
 // k_mg_ring runs levels lc .. L-1 -- down sweeps, restrictions, bottom smoothing,

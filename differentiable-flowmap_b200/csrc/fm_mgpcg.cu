@@ -1555,7 +1555,8 @@ struct fm_mgpcg {
   int lc;                      // levels lc .. L-1 run as one cluster launch (<= 0: per-level launches)
   int nc;                      // CTAs in that cluster
   size_t coarse_smem;
-  ClArgs coarse;               // its geometry: k_mg_coarse (3D FP32) ...
+  bool push;                   // which kernel: k_mg_coarse ...
+  ClArgs coarse;
   RingArgs ring;               // ... or k_mg_ring
   ClArgs* d_coarse;
   int pcg_nc;                  // CTAs of the cluster that runs a whole solve (0: the solve is a sequence of launches)
@@ -1576,9 +1577,16 @@ constexpr int kCoarseMaxNC = 8;
 constexpr long kCoarseMaxPairs = 2 * kClThreads;
 static_assert(kRingThreads == kClThreads && kRingPPT == 2, "one rule for both kernels");
 
-// Which kernel that is (fm_mg_ring.cuh has the figures).
+// Which kernel that is: k_mg_coarse in 3D FP32, k_mg_ring in 3D FP64 (fm_mg_ring.cuh has the figures).  In 2D the ring,
+// unless the coarsest level is so large that its sweeps decide and its rows are multiples of 32 cells, whose
+// natural order meets bank conflicts (V-cycles on four levels, us, ring / push: FP32 512^2 and 448x512 84.3 / 78.1, 83.0 /
+// 78.4, without such rows 384^2 74.4 / 74.9, 416^2 81.1 / 81.5; FP64 256^2 68.5 / 65.1,
+// 512x256 79.5 / 74.7, without 304^2 79.9 / 81.9).  In FP64 the push kernel takes only one pair a thread in
+// registers (384^2 83.0 / 104.9).
 template <typename T, int D>
-constexpr bool kPushCoarse = D == 3 && sizeof(T) == 4;
+constexpr bool kCanPush = D == 2 || sizeof(T) == 4;
+template <typename T, int D>
+constexpr bool kCanRing = D == 2 || sizeof(T) == 8;
 
 static long coarse_pairs(const Shape& s, int dim, int planes) {
   const long nin = dim == 3 ? s.s2 : s.s1;
@@ -1612,7 +1620,16 @@ static size_t ring_layout(RingArgs& a, const fm_mgpcg* S, int lc, int nc, size_t
 }
 
 template <typename T, int D>
+static bool push_coarse(const fm_mgpcg* S) {
+  if (D == 3) return kCanPush<T, D>;
+  const Shape& b = S->lv[S->L - 1];
+  const long pairs = coarse_pairs(b, D, b.s0);
+  return b.s1 % 32 == 0 && pairs >= 512 && pairs <= (sizeof(T) == 4 ? kCoarseMaxPairs : (long)kClThreads);
+}
+
+template <typename T, int D>
 static void plan_coarse(fm_mgpcg* S) {
+  S->push = push_coarse<T, D>(S);
   S->lc = -1;
   S->nc = 0;
   S->coarse_smem = 0;
@@ -1623,9 +1640,9 @@ static void plan_coarse(fm_mgpcg* S) {
     if (t.s0 % (2 * nc) != 0 || coarse_pairs(t, D, t.s0 / nc) > kCoarseMaxPairs) continue;
     bool fits = true;
     for (int m = l + 1; m < S->L; ++m) fits = fits && coarse_pairs(S->lv[m], D, S->lv[m].s0) <= kCoarseMaxPairs;
-    const size_t smem = kPushCoarse<T, D> ? cl_layout(S->coarse, S->lv, l, l + 1, S->L, D, sizeof(T), nc, false, false)
-                                          : ring_layout(S->ring, S, l, nc, sizeof(T));
-    if (!fits || smem == 0 || smem > (kPushCoarse<T, D> ? kClMaxSmem : 200 * 1024)) continue;
+    const size_t smem = S->push ? cl_layout(S->coarse, S->lv, l, l + 1, S->L, D, sizeof(T), nc, false, false)
+                                : ring_layout(S->ring, S, l, nc, sizeof(T));
+    if (!fits || smem == 0 || smem > (S->push ? kClMaxSmem : 200 * 1024)) continue;
     S->lc = l;
     S->nc = nc;
     S->coarse_smem = smem;
@@ -1641,24 +1658,25 @@ static void plan_coarse(fm_mgpcg* S) {
 // 16 CTAs instead of 8, FP32, a 128^3 projection: 443 -> 434 us.
 template <typename T, int D>
 static bool enable_coarse(fm_mgpcg* S) {
-  if constexpr (kPushCoarse<T, D>) {
-    const Shape t = S->lv[S->lc];
-    const int nc = 2 * kCoarseMaxNC;
-    if (S->nc == kCoarseMaxNC && t.s0 % (2 * nc) == 0 && coarse_pairs(t, D, t.s0 / S->nc) > kClThreads) {
-      ClArgs a = S->coarse;
-      const size_t smem = cl_layout(a, S->lv, S->lc, S->lc + 1, S->L, D, sizeof(T), nc, false, false);
-      if (smem > 0 && smem <= kClMaxSmem && cl_enable(k_mg_coarse<T, D, DevState>, nc, smem)) {
-        S->coarse = a;
-        S->nc = nc;
-        S->coarse_smem = smem;
-        return true;
+  if constexpr (kCanPush<T, D>)
+    if (S->push) {
+      const Shape t = S->lv[S->lc];
+      const int nc = 2 * kCoarseMaxNC;
+      if (S->nc == kCoarseMaxNC && t.s0 % (2 * nc) == 0 && coarse_pairs(t, D, t.s0 / S->nc) > kClThreads) {
+        ClArgs a = S->coarse;
+        const size_t smem = cl_layout(a, S->lv, S->lc, S->lc + 1, S->L, D, sizeof(T), nc, false, false);
+        if (smem > 0 && smem <= kClMaxSmem && cl_enable(k_mg_coarse<T, D, DevState>, nc, smem)) {
+          S->coarse = a;
+          S->nc = nc;
+          S->coarse_smem = smem;
+          return true;
+        }
+        cudaGetLastError();
       }
-      cudaGetLastError();
+      return raise_smem_limit(k_mg_coarse<T, D, DevState>, S->coarse_smem);
     }
-    return raise_smem_limit(k_mg_coarse<T, D, DevState>, S->coarse_smem);
-  } else {
-    return raise_smem_limit(k_mg_ring<T, D>, S->coarse_smem);
-  }
+  if constexpr (kCanRing<T, D>) return raise_smem_limit(k_mg_ring<T, D>, S->coarse_smem);
+  return false;
 }
 
 // The coarse levels in one cluster launch where they fit.
@@ -1693,10 +1711,13 @@ static inline unsigned blocks_for(long n, int threads, long cap) {
 // Levels lc .. L-1 of the V-cycle as one cluster launch.
 template <typename T, int D>
 static void launch_coarse(fm_mgpcg* S, cudaStream_t s) {
-  if constexpr (kPushCoarse<T, D>) {
-    cl_launch(k_mg_coarse<T, D, DevState>, S->nc, S->coarse_smem, s, (const ClArgs*)S->d_coarse, (const T*)S->r[S->lc],
-              (T*)S->z[S->lc], (const DevState*)S->st);
-  } else {
+  if constexpr (kCanPush<T, D>)
+    if (S->push) {
+      cl_launch(k_mg_coarse<T, D, DevState>, S->nc, S->coarse_smem, s, (const ClArgs*)S->d_coarse, (const T*)S->r[S->lc],
+                (T*)S->z[S->lc], (const DevState*)S->st);
+      return;
+    }
+  if constexpr (kCanRing<T, D>) {
     RingArgs a = S->ring;
     a.r_top = S->r[S->lc];
     a.z_top = S->z[S->lc];
