@@ -372,7 +372,8 @@ int fm_mgpcg_stats(fm_mgpcg *solver, void *stream, int reset, fm_mg_stats *out);
  * capacity check comes before the field-pointer check, so a call with NULL
  * fields tells whether a grid fits (FM_ERR_CAPACITY if not, FM_ERR_ARG if so).
  * Every call synchronises `stream` to poll convergence (params->check_every
- * iterations per poll; 0 means 4).  Result and status as fm_project. */
+ * iterations per poll; 0 means 4).  Status as fm_project, the result equal to rounding (a
+ * handle may solve a small grid in one launch, whose inner products add up in another order). */
 int fm_project_noalloc(const fm_grid *g, int dtype, const fm_mg_params *params, void *ux, void *uy, void *uz,
                        void *stream, int *iters, double *rtr);
 
