@@ -420,7 +420,15 @@ static void launch_fixed(const fm_grid& g, T dx, const StTerms<T>& terms, const 
       if (ti == 4) launch_fixed3<T, ORDER, 0, 4>(g, dx, terms, out, s);
       else launch_fixed3<T, ORDER, 0, 8>(g, dx, terms, out, s);
     } else {
-      if (ti == 4) launch_fixed3<T, ORDER, 1, 4>(g, dx, terms, out, s);
+      // where the passes share memory an SM holds one CTA, and a wave of tiles 4 high takes 0.7 to 0.8 of the time of
+      // one of tiles 8 high: the lower ones where their waves are sooner done (FP64 order 3, us by tiles 8 / 4 high:
+      // 35x78x31 in 2 / 2 waves 47 / 42, 24^3 in 1 / 1 33 / 25, 25x49x122 in 3 / 4 74 / 80, 40x61x90 in 3 / 6 79 / 111)
+      const auto waves = [&](int t) {
+        const long ctas = 3L * ((g.n[2] + kTK3) / kTK3) * ((g.n[1] + kTJ3) / kTJ3) * ((g.n[0] + t) / t);
+        return (ctas + 147) / 148;
+      };
+      if (ti == 4 || (!Fixed3<T, ORDER, 1, 8>::kOwnB && 5 * waves(8) > 4 * waves(4)))
+        launch_fixed3<T, ORDER, 1, 4>(g, dx, terms, out, s);
       else launch_fixed3<T, ORDER, 1, 8>(g, dx, terms, out, s);
     }
     return;
