@@ -240,13 +240,15 @@ __global__ void __launch_bounds__(kAdjThreads) k_advect_grid_adj(fm_grid g, T dx
   const long n0 = (long)blockIdx.x * blockDim.x + threadIdx.x, n = n0 < s.size() ? n0 : s.size() - 1;
   const T lam = pick(gout, slot)[n];
   // a zero adjoint contributes nothing to either gradient; its lane only keeps
-  // the warp whole for the scatters.  Whether it samples: in FP64 RK2 it does not (velocity at 64^3, us, dense
-  // and with 1 % of the adjoint not zero, without / with its samples: 183, 90 / 197, 106; RK4 402, 225 / 392,
-  // 219; FP32 the same within 1 %).  A second body for warps of few lanes, lane by lane, made the dense ones
-  // slower (FP64 164 -> 212 us at 40x61x90, RK2: instruction fetch).
+  // the warp whole for the scatters.  Whether it samples: in 3D FP64 RK2 it does
+  // not (velocity at 64^3, us, dense and with 1 % of the adjoint not zero, without /
+  // with its samples: 183, 90 / 197, 106; RK4 402, 225 / 392, 219; scalar at
+  // 250x333 RK2 9.1 / 8.4; FP32 the same within 1 %).  A second body for warps of
+  // few lanes, lane by lane, made the dense ones slower (FP64 164 -> 212 us at
+  // 40x61x90, RK2: instruction fetch).
   const bool live = n0 < s.size() && lam != (T)0;
   if (!__any_sync(0xffffffffu, live)) return;
-  constexpr bool kSkip = sizeof(T) == 8 && RK == 2;
+  constexpr bool kSkip = D == 3 && sizeof(T) == 8 && RK == 2;
   const bool samples = !kSkip || live;
   int i, j, k;
   unflatten(s, n, i, j, k);
